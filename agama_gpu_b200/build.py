@@ -15,6 +15,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -24,9 +25,9 @@ LIB = PKG / "libagb.so"
 STAMP = PKG / ".libagb.stamp"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-shared",
+NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC",
               "--expt-relaxed-constexpr", "-Xptxas", "-v"]
-SOURCES = ["eval.cu", "peak.cu"]
+SOURCES = ["eval.cu", "split.cu", "peak.cu"]
 
 
 def _nvcc() -> str:
@@ -52,13 +53,25 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     dig = _digest()
     if not force and LIB.exists() and STAMP.exists() and STAMP.read_text() == dig:
         return LIB
+    # one nvcc per source, side by side, then one link
+    objs = PKG / "build"
+    objs.mkdir(exist_ok=True)
+
+    def compile_one(src: str):
+        cmd = [_nvcc(), *ARCH, *NVCC_FLAGS, "-I", str(ROOT / "include"), "-c", str(CSRC / src),
+               "-o", str(objs / (src + ".o"))]
+        return cmd, subprocess.run(cmd, capture_output=True, text=True)
+
+    with ThreadPoolExecutor(len(SOURCES)) as pool:
+        runs = list(pool.map(compile_one, SOURCES))
     tmp = LIB.with_suffix(".so.tmp")
-    cmd = [_nvcc(), *ARCH, *NVCC_FLAGS, "-I", str(ROOT / "include"),
-           *[str(CSRC / s) for s in SOURCES], "-o", str(tmp)]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    log = res.stdout + res.stderr
-    (PKG / "build.log").write_text(" ".join(cmd) + "\n" + log)
-    if res.returncode != 0:
+    if all(r.returncode == 0 for _, r in runs):
+        cmd = [_nvcc(), *ARCH, "-shared", "-Xcompiler", "-fPIC",
+               *[str(objs / (s + ".o")) for s in SOURCES], "-o", str(tmp)]
+        runs.append((cmd, subprocess.run(cmd, capture_output=True, text=True)))
+    log = "".join(" ".join(cmd) + "\n" + r.stdout + r.stderr for cmd, r in runs)
+    (PKG / "build.log").write_text(log)
+    if any(r.returncode != 0 for _, r in runs):
         raise RuntimeError(f"nvcc failed:\n{log[-4000:]}")
     if verbose:
         print(log)

@@ -17,11 +17,17 @@
 //                   key) and a sorted AoS copy of xyz
 // Within a bin the order is not deterministic; each point's result does not
 // depend on it.
+//
+// Calls of at most AGB_BIN_SMALL points are sorted by bin_small in ONE launch: the
+// passes' launches and the gaps between them cost more than the work there.
 #pragma once
+#include <cooperative_groups.h>
 #include "agb_dev.cuh"
 
 #define AGB_BIN_TILE_MAX 4096      // points per block in passes 1 and 3 (at most)
 #define AGB_MAX_BINS 8192
+#define AGB_BIN_SMALL 32768        // most points of bin_small: 8 blocks x 1024 threads x 4
+#define AGB_BIN_SMALL_BINS 1024    // and most bins: one thread each in the scan
 
 struct BinKey {
     double sigma, g0, g1, g2;     // frame of the keyed Multipole leaf
@@ -126,5 +132,81 @@ bin_scatter(const double* __restrict__ xyz, long long n, int tile, int n_bins,
         xyz_sorted[3 * pos] = xyz[3 * i];
         xyz_sorted[3 * pos + 1] = xyz[3 * i + 1];
         xyz_sorted[3 * pos + 2] = xyz[3 * i + 2];
+    }
+}
+
+// The whole sort in one launch: a cluster of 8 blocks, each with an eighth of the points, at
+// most 4 a thread, kept in registers between counting and placing.  The blocks read each
+// other's histograms through distributed shared memory; every block scans the bins itself.
+// Bound by the latency of its steps (the log of a point's radius, two cluster barriers, the
+// scan), not by bandwidth.
+#define AGB_BIN_SMALL_BLOCKS 8
+__global__ void __cluster_dims__(AGB_BIN_SMALL_BLOCKS, 1, 1) __launch_bounds__(1024)
+bin_small(const double* __restrict__ xyz, int n, BinKey b, int n_bins, int* __restrict__ keys,
+          int* __restrict__ perm, double* __restrict__ xyz_sorted)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    __shared__ int hist[AGB_BIN_SMALL_BINS], base[AGB_BIN_SMALL_BINS], part[32];
+    const int rank = (int)cluster.block_rank(), t = threadIdx.x;
+    if (b.leaf) {                 // the leaf's frame at this call's time (agb_eval_timed)
+        b.sigma = b.leaf->sigma;
+        b.g0 = b.leaf->g0; b.g1 = b.leaf->g1; b.g2 = b.leaf->g2;
+    }
+    hist[t] = 0;
+    __syncthreads();
+    const int per = (n + AGB_BIN_SMALL_BLOCKS - 1) / AGB_BIN_SMALL_BLOCKS;
+    const int lo = rank * per, hi = min(lo + per, n);
+    double p[4][3];
+    int key[4], at[4];
+    #pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int i = lo + t + 1024 * j;
+        if (i >= hi) continue;
+        p[j][0] = xyz[3 * i]; p[j][1] = xyz[3 * i + 1]; p[j][2] = xyz[3 * i + 2];
+        key[j] = bin_of(b, p[j][0], p[j][1], p[j][2]);
+        at[j] = atomicAdd(&hist[key[j]], 1);
+    }
+    cluster.sync();
+    // bin t: its points in all blocks, and in the blocks before this one
+    int all = 0, before = 0;
+    if (t < n_bins) {
+        #pragma unroll
+        for (int r = 0; r < AGB_BIN_SMALL_BLOCKS; ++r) {
+            const int v = *cluster.map_shared_rank(&hist[t], r);
+            all += v;
+            if (r < rank) before += v;
+        }
+    }
+    int inc = all;
+    #pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, d);
+        if ((t & 31) >= d) inc += v;
+    }
+    if ((t & 31) == 31) part[t >> 5] = inc;
+    __syncthreads();
+    if (t < 32) {
+        int v = part[t];
+        #pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, v, d);
+            if (t >= d) v += u;
+        }
+        part[t] = v;
+    }
+    __syncthreads();
+    base[t] = inc - all + before + (t >= 32 ? part[(t >> 5) - 1] : 0);
+    cluster.sync();               // bases complete here, histograms read everywhere
+    #pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int i = lo + t + 1024 * j;
+        if (i >= hi) continue;
+        const int pos = base[key[j]] + at[j];
+        if (perm) perm[pos] = i;
+        keys[i] = pos;
+        xyz_sorted[3 * pos] = p[j][0];
+        xyz_sorted[3 * pos + 1] = p[j][1];
+        xyz_sorted[3 * pos + 2] = p[j][2];
     }
 }

@@ -17,9 +17,8 @@
 #include <stdarg.h>
 #include <stdlib.h>
 #include "agb_dev.cuh"
-#include "multipole.cuh"
-#include "cylspline.cuh"
-#include "analytic.cuh"
+#include "eval_point.cuh"
+#include "launch.cuh"
 #include "bin.cuh"
 #include "mp_grad.cuh"
 #include "cs_grad.cuh"
@@ -58,44 +57,12 @@ static int check_launch(const char* what)
 // ---------------------------------------------------------------------------
 // the fused kernel
 // ---------------------------------------------------------------------------
-// AN: the tree holds analytic leaves only (no expansion code compiled in: a
-// small register footprint and more resident blocks for the Hessian modes)
-template <int MODE, typename R, bool EXACT, bool AN = false>
-__device__ __forceinline__ void eval_component(const DevComp& c, double x, double y, double z,
-                                               PointOut& o)
-{
-    switch (c.kind) {
-    case AGB_KIND_MULTIPOLE:     if (!AN) multipole_point<MODE, R>(c, x, y, z, o); break;
-    case AGB_KIND_CYLSPLINE:     if (!AN) cylspline_point<MODE, EXACT, R>(c, x, y, z, o); break;
-    case AGB_KIND_NFW:           nfw_point<MODE>(c.p, x, y, z, o); break;
-    case AGB_KIND_PLUMMER:       plummer_point<MODE>(c.p, x, y, z, o); break;
-    case AGB_KIND_HERNQUIST:     hernquist_point<MODE>(c.p, x, y, z, o); break;
-    case AGB_KIND_DEHNEN:        dehnen_point<MODE>(c.p, x, y, z, o); break;
-    case AGB_KIND_ISOCHRONE:     isochrone_point<MODE>(c.p, x, y, z, o); break;
-    case AGB_KIND_MIYAMOTONAGAI: mn_point<MODE>(c.p, x, y, z, o); break;
-    case AGB_KIND_LOGHALO:       loghalo_point<MODE>(c.p, x, y, z, o); break;
-    case AGB_KIND_DISKANSATZ:    diskansatz_point<MODE>(c.p, x, y, z, o); break;
-    case AGB_KIND_UNIFORMACC:    uniform_point<MODE>(c.p, x, y, z, o); break;
-    default: break;
-    }
-}
-
 // Binned calls evaluate the points in interval order.  Writing each point's
 // outputs straight to its input position scatters 8-byte stores over the whole
 // output (uncoalesced: one sector per lane per store); with room in the
 // workspace the kernel instead writes records in sorted order ("stage") and
 // unpermute_kernel gathers them back, reading one record per point and writing
 // every output array contiguously.
-// internal mode of agb_eval_vjp_force: the VJP plus the force of the same leaves
-// (written to the `hess` pointer as [N,3]) from the same per-point sums
-#define AGB_MODE_VJPF 5
-
-__host__ __device__ constexpr int stage_rec(int mode)
-{
-    return mode == AGB_MODE_HESS ? 10 : mode == AGB_MODE_GRAD ? 4 : mode == AGB_MODE_VJP ? 3
-         : mode == AGB_MODE_VJPF ? 6 : 1;
-}
-#define AGB_STAGE_MAX_REC 10
 
 template <int MODE>
 __global__ void __launch_bounds__(256)
@@ -219,101 +186,13 @@ agb_eval_kernel(const __grid_constant__ EvalArgs a)
                 }
             }
         }
-        if (VJP) {
-            // L(Phi, F): dL/dx = gPhi grad(Phi) + (dF/dx)^T gF = gPhi grad(Phi) - H gF
-            const double gp = a.gphi ? a.gphi[i] : 0.0;
-            double f0 = 0.0, f1 = 0.0, f2 = 0.0;
-            if (a.gforce) { f0 = a.gforce[3 * i]; f1 = a.gforce[3 * i + 1]; f2 = a.gforce[3 * i + 2]; }
-            const double v0 = gp * g0 - (h[0] * f0 + h[3] * f1 + h[5] * f2);
-            const double v1 = gp * g1 - (h[3] * f0 + h[1] * f1 + h[4] * f2);
-            const double v2 = gp * g2 - (h[5] * f0 + h[4] * f1 + h[2] * f2);
-            if (MODE == AGB_MODE_VJPF) {
-                if (a.stage) {
-                    double* o = a.stage + 6 * pos;
-                    o[0] = v0; o[1] = v1; o[2] = v2; o[3] = -g0; o[4] = -g1; o[5] = -g2;
-                } else {
-                    a.grad[3 * i] = v0; a.grad[3 * i + 1] = v1; a.grad[3 * i + 2] = v2;
-                    a.hess[3 * i] = -g0; a.hess[3 * i + 1] = -g1; a.hess[3 * i + 2] = -g2;
-                }
-                continue;
-            }
-            double* o = a.stage ? a.stage + 3 * pos : a.grad + 3 * i;
-            o[0] = v0; o[1] = v1; o[2] = v2;
-            continue;
-        }
-        const double sg = (a.out_flags & AGB_OUT_NEGATE) ? -1.0 : 1.0;
-        if (MODE == AGB_MODE_DENS) {
-            if (a.stage) a.stage[pos] = rho;
-            else a.rho[i] = rho;
-            continue;
-        }
-        if (a.stage) {
-            // sorted order: consecutive threads write consecutive records
-            constexpr int REC = stage_rec(MODE);
-            double* o = a.stage + REC * pos;
-            o[0] = phi;
-            if (MODE != AGB_MODE_POT) { o[1] = sg * g0; o[2] = sg * g1; o[3] = sg * g2; }
-            if (MODE == AGB_MODE_HESS) {
-                #pragma unroll
-                for (int q = 0; q < 6; ++q) o[4 + q] = sg * h[q];
-            }
-            continue;
-        }
-        if (a.phi) a.phi[i] = phi;
-        if (MODE != AGB_MODE_POT && a.grad) {
-            a.grad[3 * i] = sg * g0; a.grad[3 * i + 1] = sg * g1; a.grad[3 * i + 2] = sg * g2;
-        }
-        if (MODE == AGB_MODE_HESS) {
-            #pragma unroll
-            for (int q = 0; q < 6; ++q) a.hess[6 * i + q] = sg * h[q];
-        }
+        eval_write<MODE>(a, pos, i, phi, g0, g1, g2, h, rho);
     }
 }
 
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-// Values fixed for the life of a device (its SM count, the resident blocks of one
-// kernel) are read on the device current at the call and cached per device index.
-// Host threads making their first call at the same time store the same value, so
-// relaxed atomics are enough.
-#define AGB_MAX_DEVICES 64
-
-static int current_device()
-{
-    int d = 0;
-    if (cudaGetDevice(&d) != cudaSuccess || d < 0 || d >= AGB_MAX_DEVICES) d = 0;
-    return d;
-}
-
-static std::atomic<int> g_num_sms[AGB_MAX_DEVICES];
-
-static int num_sms()
-{
-    const int dev = current_device();
-    int v = g_num_sms[dev].load(std::memory_order_relaxed);
-    if (v == 0) {
-        if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0)
-            v = 148;
-        g_num_sms[dev].store(v, std::memory_order_relaxed);
-    }
-    return v;
-}
-
-// resident blocks per SM of `kernel` at `threads` threads, cached per device in `cache`
-template <typename K>
-static int blocks_per_sm(std::atomic<int>* cache, K kernel, int threads)
-{
-    const int dev = current_device();
-    int b = cache[dev].load(std::memory_order_relaxed);
-    if (b == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, threads, 0) != cudaSuccess || b < 1)
-            b = 1;
-        cache[dev].store(b, std::memory_order_relaxed);
-    }
-    return b;
-}
-
 static int grid_for(long long n)
 {
     const long long blocks = (n + 255) / 256;
@@ -440,6 +319,7 @@ static int launch_mode(int mode, int precision, EvalArgs& a, cudaStream_t st)
 static int launch_eval_mode(int mode, int precision, EvalArgs& a, cudaStream_t st)
 {
     const bool mixed = precision == AGB_PREC_MIXED;
+    if (agb_launch_split(mode, mixed, a, st)) return check_launch("agb_split_kernel");
     if (a.dleaves) {        // leaves computed on the device (agb_eval_timed)
         switch (mode) {
         case AGB_MODE_POT:  mixed ? launch_eval<AGB_MODE_POT, float, false, true>(a, st)  : launch_eval<AGB_MODE_POT, double, false, true>(a, st); break;
@@ -528,13 +408,43 @@ struct BinPlan {
     int leaf;          // the keyed leaf
 };
 
+// What a point gains (ns) when the walk of this Multipole reads its records as broadcasts
+// instead of one row per lane.  The lanes' rows lie n_lm records of 48 bytes apart: rows that
+// fall on the same 16 bytes of a 128-byte line queue up in L1, so it depends on how many
+// different offsets the stride gives (1 to 8).  Measured, FP64 forces of 1M-4M points, sorted
+// against unsorted without the sort's cost (ns; harmonics, offsets): 0.09 (28, 2), 0.03
+// (45, 8), 0.06 (49, 8), 0.58 (64, 1), 0.13 (66, 4), 0.11 (81, 8), 0.11 (91, 8), 1.06 (144, 1);
+// with tables larger than the L1s 0.27 (153, 8), 1.2 (561, 8).  Mixed precision gains about
+// two thirds, the potential alone nearly twice as much.
+static double sort_gain(const agb_component& c, int mode)
+{
+    int offsets = 8;
+    for (int q = 8; q > 1 && (c.n_lm * 48 / 16) % (16 / q) == 0; q >>= 1) offsets = q / 2;
+    const double l2 = 48.0 * c.n_lm * c.n_int > 400e3 ? 0.8e-3 : 0.0;
+    return c.n_lm * (6.5e-3 / offsets + 0.5e-3 + l2) * (mode == AGB_MODE_POT ? 1.7 : 1.0);
+}
+
+// Whether sorting n points pays: the sort and the gather of the outputs cost 13 us, or 5 us
+// in one launch (bin_small), and 0.06 ns a point (0.16 with Hessians); half of the 13 us are
+// gained back by the kernel's coalesced stores and warmer rows, so the line lies at 6 us.
+// E.g. FP64 forces, sorted / unsorted: lmax 8 44 / 32 us at 100k points; lmax 12 103 / 108 at
+// 300k; lmax 16 45 / 46 us at 40k, 75 / 90 at 100k, 1490 / 2365 at 4M.  mode < 0: any mode
+// (workspace sizes).
+static bool sort_pays(double gain, int64_t n, int n_bins, int mode)
+{
+    const bool small = n <= AGB_BIN_SMALL && n_bins <= AGB_BIN_SMALL_BINS;
+    const double cost = mode == AGB_MODE_HESS ? 0.16 : 0.06;
+    return (double)n * (gain - cost) > (small ? 5000.0 : 6000.0);
+}
+
+// eval: an evaluation in `mode` (else an adjoint or table gradient, whose sums need the order)
 static BinPlan plan_binning(const agb_component* comps, const agb_leaf* leaves, int n_leaves,
-                            int64_t n, int out_flags)
+                            int64_t n, int out_flags, int eval = 0, int mode = -1)
 {
     BinPlan b;
     memset(&b, 0, sizeof(b));
     if ((out_flags & AGB_OUT_NO_BINNING) || n > 0x7fffffffLL) return b;
-    if (n < AGB_BIN_MIN_POINTS && !(out_flags & AGB_OUT_BIN_ALWAYS)) return b;
+    if (!eval && n < AGB_BIN_MIN_POINTS && !(out_flags & AGB_OUT_BIN_ALWAYS)) return b;
     int best = -1, best_lm = 0;
     for (int L = 0; L < n_leaves; ++L) {
         const agb_component& c = comps[leaves[L].comp];
@@ -545,6 +455,16 @@ static BinPlan plan_binning(const agb_component* comps, const agb_leaf* leaves, 
     }
     if (best < 0 || best_lm < 2) return b;
     const agb_component& c = comps[leaves[best].comp];
+    if (eval && !(out_flags & AGB_OUT_BIN_ALWAYS)) {
+        double gain = 0.0;            // of every Multipole in the keyed one's frame
+        for (int L = 0; L < n_leaves; ++L) {
+            const agb_component& q = comps[leaves[L].comp];
+            if (q.kind == AGB_KIND_MULTIPOLE && leaves[L].sigma == leaves[best].sigma &&
+                !memcmp(leaves[L].gamma, leaves[best].gamma, sizeof(leaves[L].gamma)))
+                gain += sort_gain(q, mode < 0 ? AGB_MODE_POT : mode);
+        }
+        if (!sort_pays(gain, n, c.n_int + 2, mode)) return b;
+    }
     b.on = true;
     b.leaf = best;
     b.key.sigma = leaves[best].sigma;
@@ -561,8 +481,6 @@ static BinPlan plan_binning(const agb_component* comps, const agb_leaf* leaves, 
     b.n_bins = (int)((n + (1LL << lb) - 1) >> lb) * nb;
     return b;
 }
-
-static constexpr size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 static size_t ws_bytes(const BinPlan& b, int64_t n)
 {
@@ -674,6 +592,13 @@ static int run_binning(EvalArgs& a, const BinPlan& b, const double* xyz, int64_t
         cudaFuncSetAttribute(bin_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * AGB_MAX_BINS);
         g_bin_attr_set.fetch_or(bit, std::memory_order_release);
     }
+    if (n <= AGB_BIN_SMALL && b.n_bins <= AGB_BIN_SMALL_BINS) {
+        bin_small<<<AGB_BIN_SMALL_BLOCKS, 1024, 0, st>>>(xyz, (int)n, b.key, b.n_bins, keys,
+                                                         with_perm ? perm : nullptr, xs);
+        a.xyz = xs;
+        a.perm = with_perm ? perm : nullptr;
+        return check_launch("bin_small");
+    }
     if (cudaMemsetAsync(counts, 0, 4 * (size_t)b.n_bins, st) != cudaSuccess)
         return set_err(AGB_ERR_DEVICE, "agb_eval: memset of bin counts failed");
     // points per block: the largest power of two from 512 to 4096 that still gives
@@ -717,11 +642,11 @@ static int eval_impl(const agb_component* comps, int n_comps, const agb_leaf* le
     a.gphi = g_vjp_phi; a.gforce = g_vjp_force;
     if ((rc = pack_args(a, comps, n_comps, leaves, n_leaves, precision))) return rc;
 
-    const BinPlan b = plan_binning(comps, leaves, n_leaves, n, out_flags);
+    const BinPlan b = plan_binning(comps, leaves, n_leaves, n, out_flags, 1, mode);
     // sorted-order output staging when the workspace has room for it (always for
     // agb_eval's own allocation and for workspaces sized by agb_eval_workspace_bytes)
     const size_t staged = ws_bytes_staged(b, n);
-    const bool stage = b.on && (own_ws || (workspace && workspace_bytes >= staged));
+    const bool stage = b.on && n > AGB_BIN_SMALL && (own_ws || (workspace && workspace_bytes >= staged));
     const size_t need = stage ? staged : ws_bytes(b, n);
     void* ws = workspace;
     if (need) {
@@ -759,7 +684,7 @@ extern "C" size_t agb_eval_workspace_bytes(const agb_component* comps, int n_com
     if (!comps || !leaves || n_leaves < 1 || n_comps < 1) return 0;
     for (int L = 0; L < n_leaves; ++L)
         if (leaves[L].comp < 0 || leaves[L].comp >= n_comps) return 0;
-    return ws_bytes_staged(plan_binning(comps, leaves, n_leaves, n, out_flags), n);
+    return ws_bytes_staged(plan_binning(comps, leaves, n_leaves, n, out_flags, 1), n);
 }
 
 extern "C" int64_t agb_eval_wave_points(const agb_component* comps, int n_comps,
@@ -1087,7 +1012,7 @@ extern "C" size_t agb_eval_timed_workspace_bytes(const agb_component* comps, int
         if (p->max_comp[i] >= n_comps) return 0;
     agb_leaf lv[AGB_MAX_LEAVES];
     tp_template_leaves(p, lv);
-    return TP_LEAF_BYTES + ws_bytes_staged(plan_binning(comps, lv, p->n, n, out_flags), n);
+    return TP_LEAF_BYTES + ws_bytes_staged(plan_binning(comps, lv, p->n, n, out_flags, 1), n);
 }
 
 extern "C" int agb_eval_timed(const agb_component* comps, int n_comps, const agb_time_plan* p,
@@ -1135,7 +1060,7 @@ extern "C" int agb_eval_timed(const agb_component* comps, int n_comps, const agb
     if ((rc = launch_time_leaves(p, pair, step, t0, dt, off, dl, st))) return rc;
     char* ws = (char*)workspace + TP_LEAF_BYTES;
     const size_t room = workspace_bytes - TP_LEAF_BYTES;
-    BinPlan b = plan_binning(comps, lv, p->n, n, out_flags);
+    BinPlan b = plan_binning(comps, lv, p->n, n, out_flags, 1, mode);
     if (b.on) {
         b.key.leaf = dl + b.leaf;
         const size_t staged = ws_bytes_staged(b, n);
@@ -1144,7 +1069,7 @@ extern "C" int agb_eval_timed(const agb_component* comps, int n_comps, const agb
             return set_err(AGB_ERR_ARG, "agb_eval_timed: workspace of %zu bytes is smaller than "
                            "the %zu bytes agb_eval_timed_workspace_bytes asks for",
                            workspace_bytes, need + TP_LEAF_BYTES);
-        const bool stage = room >= staged;
+        const bool stage = n > AGB_BIN_SMALL && room >= staged;
         const bool vjp = mode == AGB_MODE_VJP || mode == AGB_MODE_VJPF;
         if ((rc = run_binning(a, b, xyz, n, ws, st, !stage || vjp))) return rc;
         if (stage) {

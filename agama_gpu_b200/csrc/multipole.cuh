@@ -337,6 +337,39 @@ __device__ __forceinline__ void mp_col_finish(MPCol<R>& g, R inv_sth, R q1, R np
         g.VRR *= R(2);                                          // the FP32 walk sums C''/2
 }
 
+// One |m| group's sums combined with cos/sin(m phi), and the rotation to the next m, with
+// their roundings spelled out.  The Hessian walks use them (and mp_hess_end below): a
+// Hessian near the pole cancels terms of 1/sin(theta)^2, so kernels that are to agree in it
+// (one thread per point, batches, a block per tile) must round alike.
+__device__ __forceinline__ void mp_rotate(double& cm, double& sm, double cph, double sph)
+{
+    const double t = fma(cm, cph, -__dmul_rn(sm, sph));
+    sm = fma(sm, cph, __dmul_rn(cm, sph));
+    cm = t;
+}
+
+template <typename R>
+__device__ __forceinline__ void mp_combine_hess(MPSums& t, const MPCol<R>& gc, const MPCol<R>& gs,
+                                                int m, double cm, double sm)
+{
+    const double md = (double)m;
+    const double dTc = -md * sm, dTs = md * cm;
+    auto add = [](double& s, R c, R v, double tc, double ts) {
+        s = __dadd_rn(s, fma((double)v, ts, __dmul_rn((double)c, tc)));
+    };
+    add(t.A, gc.V, gs.V, cm, sm);
+    add(t.B, gc.VR, gs.VR, cm, sm);
+    add(t.D, gc.VRR, gs.VRR, cm, sm);
+    add(t.Th, gc.VT, gs.VT, cm, sm);
+    add(t.Pos, gc.VP, gs.VP, dTc, dTs);
+    add(t.Thth, gc.VTT, gs.VTT, cm, sm);
+    add(t.BTh, gc.VRT, gs.VRT, cm, sm);
+    add(t.Ph, gc.V, gs.V, dTc, dTs);
+    t.Phph = fma(-md * md, fma((double)gs.V, sm, __dmul_rn((double)gc.V, cm)), t.Phph);
+    add(t.BPh, gc.VR, gs.VR, dTc, dTs);
+    add(t.ThPh, gc.VT, gs.VT, dTc, dTs);
+}
+
 // GEN: the interval's records come from `slab` (this interval's row of a staged
 // copy of the FP32 table, possibly in shared memory) instead of the table itself
 template <int MODE, typename R, int PAR, bool GEN = false>
@@ -346,7 +379,6 @@ __device__ __forceinline__ void mp_harmonics_reg(const DevComp& c, int k, double
                                                  const R* slab = nullptr)
 {
     constexpr bool NEED_ANG = MODE == AGB_MODE_GRAD || MODE == AGB_MODE_HESS;
-    constexpr bool NEED_ANG2 = MODE == AGB_MODE_HESS;
     const bool near_pole = sth_d < 1.0e-10;
     const R s = (R)s_d;
     R sp[6], dw[6], ew[6];
@@ -365,9 +397,13 @@ __device__ __forceinline__ void mp_harmonics_reg(const DevComp& c, int k, double
     double cm = 1.0, sm = 0.0, sinpow = 1.0, sinpow_m1 = 0.0;
     for (int m = 0; m <= lmax; ++m) {
         if (m > 0) {
-            const double t = cm * cph - sm * sph;
-            sm = sm * cph + cm * sph;
-            cm = t;
+            if constexpr (MODE == AGB_MODE_HESS) {
+                mp_rotate(cm, sm, cph, sph);
+            } else {
+                const double t = cm * cph - sm * sph;
+                sm = sm * cph + cm * sph;
+                cm = t;
+            }
             sinpow_m1 = sinpow;
             sinpow *= sth_d;
         }
@@ -448,25 +484,21 @@ __device__ __forceinline__ void mp_harmonics_reg(const DevComp& c, int k, double
         else walk(std::true_type());
         mp_col_finish<MODE, R>(gc, inv_sth, q1, np1, cot, m2);
         mp_col_finish<MODE, R>(gs, inv_sth, q1, np1, cot, m2);
+        if constexpr (MODE == AGB_MODE_HESS) {
+            mp_combine_hess<R>(tot, gc, gs, m, cm, sm);
+            continue;
+        }
         // combine the group's cos and sin sums with cos/sin(m phi) in FP64
         const double md = (double)m;
         const double dTc = -md * sm, dTs = md * cm;
         tot.A += (double)gc.V * cm + (double)gs.V * sm;
         if (MODE != AGB_MODE_POT) tot.B += (double)gc.VR * cm + (double)gs.VR * sm;
-        if (MODE == AGB_MODE_HESS || MODE == AGB_MODE_DENS)
+        if (MODE == AGB_MODE_DENS)
             tot.D += (double)gc.VRR * cm + (double)gs.VRR * sm;
         if (MODE == AGB_MODE_DENS) tot.L += (double)gc.L * cm + (double)gs.L * sm;
         if (NEED_ANG) {
             tot.Th += (double)gc.VT * cm + (double)gs.VT * sm;
             tot.Pos += (double)gc.VP * dTc + (double)gs.VP * dTs;
-        }
-        if (NEED_ANG2) {
-            tot.Thth += (double)gc.VTT * cm + (double)gs.VTT * sm;
-            tot.BTh += (double)gc.VRT * cm + (double)gs.VRT * sm;
-            tot.Ph += (double)gc.V * dTc + (double)gs.V * dTs;
-            tot.Phph += -md * md * ((double)gc.V * cm + (double)gs.V * sm);
-            tot.BPh += (double)gc.VR * dTc + (double)gs.VR * dTs;
-            tot.ThPh += (double)gc.VT * dTc + (double)gs.VT * dTs;
         }
     }
 }
@@ -726,6 +758,100 @@ __device__ __forceinline__ void mp_finish(const MPSums& t, double inv_dlogr, dou
     }
 }
 
+// The end of a point in the Hessian mode: the monopole spline's values (c0 and its two s
+// derivatives) and the sums to Phi, gradient and Hessian, every rounding spelled out (see
+// mp_combine_hess).  The chain rule over (log r, theta, phi) is formed as J^T (P J) with the
+// second derivatives of the coordinates added, the products of P and J shared by the rows.
+__device__ __forceinline__ void mp_hess_end(const MPSums& t, double inv_dlogr, double invPhi0,
+                                            int log_scaling, double c0, double c0s, double c0ss,
+                                            double px, double py, double pz, double inv_r,
+                                            double Rc, double cth, double sth, double cph,
+                                            double sph, PointOut& o)
+{
+    auto mul = [](double x, double y) { return __dmul_rn(x, y); };
+    auto add = [](double x, double y) { return __dadd_rn(x, y); };
+    const double MP0 = AGB_MUL0 * AGB_PREFACT[0];
+    const double dc0 = mul(c0s, inv_dlogr);
+    const double d2c0 = mul(mul(c0ss, inv_dlogr), inv_dlogr);
+    double F = 1.0, dF = 0.0, d2F = 0.0, mono, dmono, d2mono;
+    if (log_scaling) {
+        const double ex = exp(c0);
+        const double P0 = 1.0 / add(invPhi0, -ex);
+        const double dPdX = mul(mul(P0, P0), ex);
+        F = P0;
+        dF = mul(dPdX, dc0);
+        d2F = mul(dPdX, fma(mul(mul(dc0, dc0), P0), add(invPhi0, ex), d2c0));
+        mono = mul(MP0, F); dmono = mul(MP0, dF); d2mono = mul(MP0, d2F);
+    } else {
+        mono = mul(MP0, c0); dmono = mul(MP0, dc0); d2mono = mul(MP0, d2c0);
+    }
+    const double Bp = mul(t.B, inv_dlogr);
+    const double Dp = mul(mul(t.D, inv_dlogr), inv_dlogr);
+    o.phi = fma(F, t.A, mono);
+    const double Pr = fma(F, Bp, fma(dF, t.A, dmono));
+    const double Pth = mul(F, t.Th), Pos = mul(F, t.Pos);
+    const double inv_r2 = mul(inv_r, inv_r);
+    const double X[3] = {px, py, pz};
+    // first derivatives of log r and theta
+    const double dlr[3] = {mul(px, inv_r2), mul(py, inv_r2), mul(pz, inv_r2)};
+    const double cr = mul(cth, inv_r);
+    const double dth[3] = {mul(cr, cph), mul(cr, sph), -mul(sth, inv_r)};
+    const double pr = mul(Pos, inv_r);
+    o.g[0] = fma(Pr, dlr[0], fma(Pth, dth[0], -mul(pr, sph)));
+    o.g[1] = fma(Pr, dlr[1], fma(Pth, dth[1], mul(pr, cph)));
+    o.g[2] = fma(Pr, dlr[2], mul(Pth, dth[2]));
+
+    // second derivatives in (log r, theta, phi)
+    const double Prr = fma(F, Dp, fma(add(dF, dF), Bp, fma(d2F, t.A, d2mono)));
+    const double Pthth = mul(F, t.Thth);
+    const double Prth = fma(F, mul(t.BTh, inv_dlogr), mul(dF, t.Th));
+    const double Pph = mul(F, t.Ph);
+    const double Pphph = mul(F, t.Phph);
+    const double Prph = fma(F, mul(t.BPh, inv_dlogr), mul(dF, t.Ph));
+    const double Pthph = mul(F, t.ThPh);
+
+    const double inv_R = (Rc > 1.0e-300) ? 1.0 / Rc : 0.0;
+    const double dph[3] = {-mul(sph, inv_R), mul(cph, inv_R), 0.0};
+    const double inv_r3 = mul(inv_r2, inv_r), inv_r4 = mul(inv_r2, inv_r2);
+    const double r5z = mul(mul(3.0, pz), mul(inv_r4, inv_r));        // 3 z / r^5
+    const double inv_s = (sth > 1.0e-14) ? 1.0 / sth : 0.0;
+    const double cos3 = mul(mul(mul(cth, inv_s), inv_s), inv_s);
+    // f = cos(theta) = z / r
+    const double zr3 = mul(pz, inv_r3);
+    const double df[3] = {-mul(zr3, px), -mul(zr3, py), fma(-zr3, pz, inv_r)};
+    double pxx = 0.0, pxy = 0.0;                 // second derivatives of phi (yy = -xx)
+    if (Rc > 1.0e-14) {
+        const double iR2 = mul(inv_R, inv_R), iR4 = mul(iR2, iR2);
+        pxx = mul(mul(mul(2.0, px), py), iR4);
+        pxy = mul(mul(add(py, px), add(py, -px)), iR4);
+    }
+    double a[3], b[3], c[3];                     // rows of P J
+    #pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        a[i] = fma(Prr, dlr[i], fma(Prth, dth[i], mul(Prph, dph[i])));
+        b[i] = fma(Prth, dlr[i], fma(Pthth, dth[i], mul(Pthph, dph[i])));
+        c[i] = fma(Prph, dlr[i], fma(Pthph, dth[i], mul(Pphph, dph[i])));
+    }
+    #pragma unroll
+    for (int p = 0; p < 6; ++p) {
+        const int i = hess_i(p), j = hess_j(p);
+        const double XX = mul(X[i], X[j]);
+        // d2 log r = (delta_ij - 2 x_i x_j / r^2) / r^2
+        const double d2lr = fma(mul(-2.0, XX), inv_r4, i == j ? inv_r2 : 0.0);
+        // d2 f / dx_i dx_j = -(delta_ij z + delta_iz x_j + delta_jz x_i)/r^3 + 3 z x_i x_j / r^5
+        double q = i == j ? pz : 0.0;
+        if (i == 2) q = add(q, X[j]);
+        if (j == 2) q = add(q, X[i]);
+        const double d2f = fma(r5z, XX, -mul(q, inv_r3));
+        const double d2th = -fma(d2f, inv_s, mul(mul(df[i], df[j]), cos3));
+        const double d2ph = p == 0 ? pxx : p == 1 ? -pxx : p == 3 ? pxy : 0.0;
+        double h = fma(Pr, d2lr, fma(Pth, d2th, mul(Pph, d2ph)));
+        h = fma(dph[j], c[i], h);
+        h = fma(dth[j], b[i], h);
+        o.h[p] = fma(dlr[j], a[i], h);
+    }
+}
+
 // STAGED: the records of intervals [k0, k1] are also in `slab` (a staged copy of
 // those rows of the FP32 table, in shared memory): a point in that range reads them
 // there (FP32 walks of regular structures; other points read the table)
@@ -813,6 +939,11 @@ __device__ __forceinline__ void multipole_point(const DevComp& c, double px, dou
     // walk so that its values are not live across it (FP64 kernel 7.22 -> 6.96 ms)
     double c0, c0s, c0ss;
     mp_quintic0(c, k, s, c0, c0s, c0ss);
+    if constexpr (MODE == AGB_MODE_HESS) {
+        mp_hess_end(t, inv_dlogr, invPhi0, c.log_scaling, c0, c0s, c0ss, px, py, pz, inv_r, Rc,
+                    cth, sth, cph, sph, o);
+        return;
+    }
     const double dc0 = c0s * inv_dlogr;
     const double d2c0 = c0ss * inv_dlogr * inv_dlogr;
     double F = 1.0, dF = 0.0, d2F = 0.0, mono, dmono, d2mono;

@@ -58,7 +58,7 @@ extern "C" {
 /* output flags for agb_eval */
 #define AGB_OUT_NEGATE     1   /* write -grad (force) and -Hessian (forceDeriv layout) */
 #define AGB_OUT_NO_BINNING 2   /* evaluate the points in input order (no scratch memory) */
-#define AGB_OUT_BIN_ALWAYS 4   /* sort by interval even below AGB_BIN_MIN_POINTS points */
+#define AGB_OUT_BIN_ALWAYS 4   /* sort by interval even where it does not pay */
 #define AGB_OUT_STAGE      32  /* batches (mixed precision, pre-sorted points): each
                                   tile's interval rows of the unit's keyed Multipole are
                                   bulk-copied (TMA, cp.async.bulk) into shared memory and
@@ -91,8 +91,10 @@ extern "C" {
 #define AGB_OUT_PPT_SHIFT   16
 #define AGB_OUT_PPT(p)      (((p) & 15) << AGB_OUT_PPT_SHIFT)
 
-/* agb_eval sorts the points by the radial interval of its heaviest Multipole
-   leaf (a counting sort in device scratch) when there are at least this many */
+/* the adjoint and table-gradient entries sort the points by the radial interval of
+   the Multipole (a counting sort in device scratch) when there are at least this many;
+   the evaluation entries sort where the estimated gain of the walk exceeds the cost of
+   the sort (more points for smaller tables; AGB_OUT_BIN_ALWAYS: always) */
 #define AGB_BIN_MIN_POINTS 16384
 
 /* component kinds */
