@@ -24,6 +24,7 @@ OUT_BLOCK_SHIFT = 12
 OUT_PPT_SHIFT = 16
 MP_NCONST = 8                # agb_component.p[3..9] + pad: invPhi0, inner s U W, outer s U W
 BIN_MIN_POINTS = 16384
+NODE_VJP_MAX = 256
 
 KIND_MULTIPOLE = 1
 KIND_CYLSPLINE = 2
@@ -128,6 +129,11 @@ def _load():
         ctypes.POINTER(AgbComponent), ctypes.POINTER(AgbLeaf), ctypes.c_void_p, ctypes.c_int64,
         ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
         ctypes.c_size_t, ctypes.c_void_p]
+    lib.agb_multipole_node_vjp.restype = ctypes.c_int
+    lib.agb_multipole_node_vjp.argtypes = [
+        ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_double, ctypes.c_double,
+        ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
+        ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
     lib.agb_multipole_adjoint_workspace_bytes.restype = ctypes.c_size_t
     lib.agb_multipole_adjoint_workspace_bytes.argtypes = [
         ctypes.POINTER(AgbComponent), ctypes.POINTER(AgbLeaf), ctypes.c_int64, ctypes.c_int]
@@ -246,6 +252,7 @@ EXPORTED = [
     "agb_eval_ws", "agb_eval_workspace_bytes", "agb_eval_wave_points", "agb_eval_static", "agb_eval_vjp",
     "agb_eval_vjp_force", "agb_multipole_adjoint_force",
     "agb_multipole_table_vjp", "agb_multipole_table_vjp_workspace_bytes",
+    "agb_multipole_node_vjp",
     "agb_multipole_adjoint", "agb_multipole_adjoint_workspace_bytes", "agb_cylspline_table_vjp",
     "agb_adjoint_step", "agb_adjoint_step_workspace_bytes", "agb_adjoint_kick", "agb_reverse_drift",
     "agb_batch_create", "agb_batch_eval", "agb_batch_eval_ws", "agb_batch_workspace_bytes",

@@ -54,6 +54,10 @@ static int check_launch(const char* what)
     return AGB_OK;
 }
 
+// for the library's other sources (launch.cuh)
+int agb_set_error(int code, const char* what) { return set_err(code, "%s", what); }
+int agb_check_launch(const char* what) { return check_launch(what); }
+
 // ---------------------------------------------------------------------------
 // the fused kernel
 // ---------------------------------------------------------------------------

@@ -48,6 +48,10 @@ inline int blocks_per_sm(std::atomic<int>* cache, K kernel, int threads)
 
 constexpr size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
+// eval.cu: the thread's last error (returns code), and a launch's status, counted
+int agb_set_error(int code, const char* what);
+int agb_check_launch(const char* what);
+
 // launch-shape bits of out_flags (blocks per slot, threads per block, points per thread)
 #define AGB_OUT_SHAPE_BITS ((15 << AGB_OUT_GRID_SHIFT) | (3 << AGB_OUT_BLOCK_SHIFT) | (15 << AGB_OUT_PPT_SHIFT))
 

@@ -196,6 +196,132 @@ def multipole_consts_from_nodes(tables, phi: torch.Tensor, dphi_dr: torch.Tensor
     return torch.stack([q if torch.is_tensor(q) else zero + q for q in parts]).to(phi.device)
 
 
+def _power_slope(A: float, dA, lnr: float):
+    """s = (A - W(A e^A)) / lnr of the builder's power-law fits with its derivatives."""
+    from scipy.special import lambertw
+    ea = float(np.exp(A))
+    w = float(np.real(lambertw(A * ea, k=0 if A > -1.0 else -1)))
+    ds = (1.0 - w / (A * ea * (1.0 + w)) * ea * (1.0 + A)) / lnr
+    return (A - w) / lnr, [ds * q for q in dA]
+
+
+def consts_and_jacobian(tables, p0: np.ndarray, d0: np.ndarray):
+    """``multipole_consts_from_nodes`` in plain numbers, with its derivatives: (8,) values and
+    (8, 6), the columns d/dPhi_00 at the nodes 0, 1, n-2, n-1 and d/d(dPhi_00/dr) at the nodes
+    0 and n-1, from the l=0 node values p0 and dPhi/dr d0 (nR,)."""
+    r = np.asarray(tables.r_grid, dtype=np.float64)
+    v, J = np.zeros(8), np.zeros((8, 6))
+    tiny = 100.0 * _EPS
+    # inner fit: columns (P1, P2, d1) = (0, 1, 4)
+    P1, P2, d1, d2 = float(p0[0]), float(p0[1]), float(d0[0]), float(d0[1])
+    r1, r2 = float(r[0]), float(r[1])
+    lnr = float(np.log(r2 / r1))
+    g1 = r1 * d1
+    v[3], J[3, 0] = P1, 1.0
+    A = np.inf
+    if tables.log_scaling and not (g1 == 0.0 or abs(P1 - P2) < tiny * max(abs(P1), abs(P2))):
+        A = lnr * g1 / (P1 - P2)
+    if np.isfinite(A) and A < 0.0:
+        s, ds = 0.0, [0.0, 0.0, 0.0]
+        if abs(A + 1.0) >= np.sqrt(_EPS):
+            s, ds = _power_slope(A, (-A / (P1 - P2), A / (P1 - P2), lnr * r1 / (P1 - P2)), lnr)
+        if not np.isfinite(s):
+            s, ds = 2.0, [0.0, 0.0, 0.0]
+        if s != 0.0:
+            U = g1 / s
+            W = (g1 - s * P1) / (-s)
+            dU = [-U / s * q for q in ds]
+            dU[2] += r1 / s
+            dW = [(1.0 if i == 0 else 0.0) - q for i, q in enumerate(dU)]
+            pred_pow = U * s * float(np.exp(s * lnr)) / r2
+        else:
+            U, W, dU, dW = g1, P1, [0.0, 0.0, r1], [1.0, 0.0, 0.0]
+            pred_pow = g1 / r2
+        pred_cub = (r2 / r1 * (6.0 * r1 * (P2 - P1) / (r2 - r1) - d1 * (2 * r1 + r2))) / (2 * r2 + r1)
+        if abs(d2 - pred_cub) < abs(d2 - pred_pow):
+            s, ds = 2.0, [0.0, 0.0, 0.0]
+            U = 0.5 * g1
+            W = P1 - U
+            dU, dW = [0.0, 0.0, 0.5 * r1], [1.0, 0.0, -0.5 * r1]
+        at = [0, 1, 4]
+        v[1], v[2], v[3] = s, U, W
+        J[1, at], J[2, at], J[3, at] = ds, dU, dW
+        if s > 0.0:
+            inv = 1.0 / W
+            if not np.any(p0 * inv >= 1.0):
+                v[0] = inv
+                J[0, at] = [-inv * inv * q for q in dW]
+    # outer fit in (eps, T, S): columns (P1, P2, d1) = (3, 2, 5)
+    P1, P2, d1 = float(p0[-1]), float(p0[-2]), float(d0[-1])
+    r1, r2 = float(r[-1]), float(r[-2])
+    lnr = float(np.log(r2 / r1))
+    at = [3, 2, 5]
+    num1, num2, den1, den2 = r1 * d1, -P1, P1, P2 * float(np.exp(lnr))
+    roundoff = (abs(num1 - num2) < max(abs(num1), abs(num2)) * tiny or
+                abs(den1 - den2) < max(abs(den1), abs(den2)) * tiny)
+    A = np.inf
+    if np.isfinite(P1) and not roundoff and den1 != den2:
+        A = lnr * (num1 - num2) / (den1 - den2)
+    if not (np.isfinite(A) and A < 0.0):
+        v[4], v[5], v[6] = 1.0, 0.0, P1
+        J[6, 3] = 1.0
+        return v, J
+    s, ds = -1.0, [0.0, 0.0, 0.0]
+    if abs(A + 1.0) >= np.sqrt(_EPS):
+        N, D = num1 - num2, den1 - den2
+        s, ds = _power_slope(A, (lnr * (1.0 / D - N / (D * D)),
+                                 lnr * N * float(np.exp(lnr)) / (D * D), lnr * r1 / D), lnr)
+        s -= 1.0
+    if not np.isfinite(s) or s >= 0.0:
+        s, ds = -2.0, [0.0, 0.0, 0.0]
+    v[4] = s + 1.0
+    J[4, at] = ds
+    if v[4] != 0.0:
+        v[5], v[6] = r1 * d1 + P1, P1
+        J[5, at], J[6, 3] = [1.0, 0.0, r1], 1.0
+    else:
+        v[6] = r1 * d1 + 2.0 * P1
+        J[6, at] = [2.0, 0.0, r1]
+    return v, J
+
+
+def _node_vjp_cuda(tables, grad_poly: torch.Tensor, nodes, grad_const: Optional[torch.Tensor]):
+    """(dL/dPhi, dL/d(dPhi/dr)) in the builder's order by the transposed builder on the GPU
+    (agb_multipole_node_vjp)."""
+    from . import _lib
+    dev = grad_poly.device
+    # the builder's own node tables, once per device
+    held = tables.__dict__.setdefault("_on_device", {})
+    if dev not in held:
+        held[dev] = [torch.tensor(np.ascontiguousarray(a), dtype=torch.float64, device=dev)
+                     for a in (tables.r_grid, tables.node_phi, tables.node_dphi_dr)]
+    r, phi, dphi = held[dev]
+    if nodes is not None:
+        phi, dphi = (q.detach().to(dev, torch.float64).contiguous() for q in nodes)
+    inv, jac, gc = float(tables.invPhi0), None, None
+    if grad_const is not None:
+        if int(np.asarray(tables.node_cols)[0]) != 0:
+            raise ValueError("the builder's l=0 column must be the coefficient file's first column")
+        if nodes is None:
+            p0, d0 = tables.node_phi[:, 0], tables.node_dphi_dr[:, 0]
+        else:
+            p0, d0 = torch.stack([phi[:, 0], dphi[:, 0]]).cpu().numpy()
+        v, jac = consts_and_jacobian(tables, np.ascontiguousarray(p0), np.ascontiguousarray(d0))
+        inv = float(v[0])
+        jac = np.ascontiguousarray(jac)
+        gc = grad_const.to(device=dev, dtype=torch.float64).contiguous()
+    g = grad_poly.to(torch.float64).contiguous()
+    out = torch.zeros((2,) + tuple(phi.shape), dtype=torch.float64, device=dev)
+    with torch.cuda.device(dev):
+        rc = _lib.lib.agb_multipole_node_vjp(
+            phi.shape[0], phi.shape[1], int(bool(tables.log_scaling)), float(tables.dlogr), inv,
+            g.data_ptr(), r.data_ptr(), phi.data_ptr(), dphi.data_ptr(),
+            None if gc is None else gc.data_ptr(), None if jac is None else jac.ctypes.data,
+            out[0].data_ptr(), out[1].data_ptr(), torch.cuda.current_stream(dev).cuda_stream)
+    _lib.check(rc, "agb_multipole_node_vjp")
+    return out[0], out[1]
+
+
 def multipole_poly_from_nodes(tables, phi: torch.Tensor, dphi_dr: torch.Tensor,
                               inv=None) -> torch.Tensor:
     """Quintic coefficients (n_lm, n_int, 6) from node tables (nR, n_lm) in the
@@ -222,22 +348,9 @@ def multipole_poly_from_nodes(tables, phi: torch.Tensor, dphi_dr: torch.Tensor,
     return quintic_poly_torch(logr, f, df, float(tables.dlogr))
 
 
-def node_vjp(tables, grad_poly: torch.Tensor, n_file_cols: Optional[int],
-             nodes=None, grad_const: Optional[torch.Tensor] = None
-             ) -> Tuple[torch.Tensor, torch.Tensor]:
-    """Carry dL/dpoly back to the node tables in the coefficient file's column order.
-
-    Returns (dL/dPhi_nodes, dL/d(dPhi/dr)_nodes), each (nR, n_file_cols); columns
-    the table builder pruned (all-zero) get zero (build with prune_threshold=0
-    to differentiate every harmonic).  n_file_cols=None returns them in the
-    builder's harmonic order instead, (nR, n_lm) like ``tables.node_phi``.
-    ``nodes`` = (phi, dphi_dr) in the builder's order when the tables were
-    replaced on the device (set_node_tables), else the builder's own node values
-    are used.  grad_const (8,): the explicit gradient with respect to invPhi0 and
-    the extrapolation constants (the kernels' g_const); with it the builder's
-    scalars are functions of the nodes (the derivative of the whole builder, as
-    set_node_tables rebuilds them), without it they are held fixed.
-    """
+def _node_vjp_torch(tables, grad_poly: torch.Tensor, nodes, grad_const: Optional[torch.Tensor]):
+    """node_vjp in the builder's order through the differentiable restatement (CPU tensors,
+    grids of more nodes than the kernel takes)."""
     dev = grad_poly.device
     if nodes is None:
         phi = torch.tensor(tables.node_phi, dtype=torch.float64, device=dev, requires_grad=True)
@@ -261,10 +374,35 @@ def node_vjp(tables, grad_poly: torch.Tensor, n_file_cols: Optional[int],
                 allow_unused=True)
             gphi = torch.zeros_like(phi) if gphi is None else gphi
             gdphi = torch.zeros_like(dphi) if gdphi is None else gdphi
+    return gphi, gdphi
+
+
+def node_vjp(tables, grad_poly: torch.Tensor, n_file_cols: Optional[int],
+             nodes=None, grad_const: Optional[torch.Tensor] = None
+             ) -> Tuple[torch.Tensor, torch.Tensor]:
+    """Carry dL/dpoly back to the node tables in the coefficient file's column order.
+
+    Returns (dL/dPhi_nodes, dL/d(dPhi/dr)_nodes), each (nR, n_file_cols); columns
+    the table builder pruned (all-zero) get zero (build with prune_threshold=0
+    to differentiate every harmonic).  n_file_cols=None returns them in the
+    builder's harmonic order instead, (nR, n_lm) like ``tables.node_phi``.
+    ``nodes`` = (phi, dphi_dr) in the builder's order when the tables were
+    replaced on the device (set_node_tables), else the builder's own node values
+    are used.  grad_const (8,): the explicit gradient with respect to invPhi0 and
+    the extrapolation constants (the kernels' g_const); with it the builder's
+    scalars are functions of the nodes (the derivative of the whole builder, as
+    set_node_tables rebuilds them), without it they are held fixed.
+    """
+    dev = grad_poly.device
+    from ._lib import NODE_VJP_MAX
+    if dev.type == "cuda" and 2 <= tables.n_int + 1 <= NODE_VJP_MAX and not tables.resampled:
+        gphi, gdphi = _node_vjp_cuda(tables, grad_poly, nodes, grad_const)
+    else:
+        gphi, gdphi = _node_vjp_torch(tables, grad_poly, nodes, grad_const)
     if n_file_cols is None:
         return gphi, gdphi
     cols = torch.as_tensor(np.asarray(tables.node_cols), dtype=torch.long, device=dev)
-    out_p = torch.zeros((phi.shape[0], n_file_cols), dtype=torch.float64, device=dev)
+    out_p = torch.zeros((gphi.shape[0], n_file_cols), dtype=torch.float64, device=dev)
     out_d = torch.zeros_like(out_p)
     out_p[:, cols] = gphi
     out_d[:, cols] = gdphi

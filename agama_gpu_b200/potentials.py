@@ -625,11 +625,8 @@ class _GPUPotBase:
                 out[comp] = out[comp] + g if comp in out else g
                 continue
             comp = key
-            cols = torch.from_numpy(comp._col_of).to(g.device)
             # the fused adjoint differentiates the rescaled table: back to the builder's
-            scale = torch.from_numpy(comp._col_scale).to(g.device)
-            g = g * scale[None, :, None]
-            gp = g.index_select(1, cols).permute(1, 0, 2).contiguous()
+            gp = comp._builder_order(g, scaled=True)
             out[comp] = out[comp] + gp if comp in out else gp
         return out
 
@@ -1110,7 +1107,18 @@ class MultipolePotentialGPU(_Component):
                 g.data_ptr(), ptr(const_grad), ptr(ws), nws,
                 ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
             _lib.check(rc, "agb_multipole_table_vjp")
-        cols = torch.from_numpy(self._col_of).to(dev)
+        return self._builder_order(g)
+
+    def _builder_order(self, g: torch.Tensor, scaled: bool = False) -> torch.Tensor:
+        """(n_lm, n_int, 6) in the builder's harmonic order from a device-layout gradient
+        (n_int, n_cols, 6); scaled: of the rescaled table, whose columns' factors apply."""
+        held = self.__dict__.setdefault("_order_dev", {})
+        if g.device not in held:
+            held[g.device] = (torch.from_numpy(self._col_of).to(g.device),
+                              torch.from_numpy(self._col_scale).to(g.device))
+        cols, scale = held[g.device]
+        if scaled:
+            g = g * scale[None, :, None]
         return g.index_select(1, cols).permute(1, 0, 2).contiguous()
 
     def node_gradients(self, grad_poly: torch.Tensor, grad_const: Optional[torch.Tensor] = None):

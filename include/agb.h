@@ -301,6 +301,23 @@ int agb_multipole_table_vjp(const agb_component* comp, const agb_leaf* leaf,
                             void* workspace, size_t workspace_bytes, void* stream);
 
 /*
+ * The coefficient gradient of a Multipole carried back to its node tables: the transpose of
+ * the table builder (log-scaling, quintic spline, coefficients).  g_poly [n_lm][n_nodes-1][6]
+ * dL/d(coefficient), harmonic-major, the builder's harmonic order; r [n_nodes]; phi, dphi
+ * [n_nodes][n_lm] the node values and dPhi/dr; dlogr, log_scaling and inv (= invPhi0 at these
+ * nodes) as the builder has them.  g_const (NULL, or AGB_MP_NCONST doubles): the explicit
+ * gradient with respect to the builder's scalars, carried on through jacobian, a HOST array
+ * [AGB_MP_NCONST][6]: their derivatives with respect to Phi_00 at the nodes 0, 1, n-2, n-1 and
+ * dPhi_00/dr at the nodes 0, n-1.  g_phi, g_dphi [n_nodes][n_lm] must be zero on entry.
+ * At most AGB_NODE_VJP_MAX nodes.  FP64.  No counterpart in the reference.
+ */
+#define AGB_NODE_VJP_MAX 256
+int agb_multipole_node_vjp(int n_nodes, int n_lm, int log_scaling, double dlogr, double inv,
+                           const double* g_poly, const double* r, const double* phi,
+                           const double* dphi, const double* g_const, const double* jacobian,
+                           double* g_phi, double* g_dphi, void* stream);
+
+/*
  * Fused adjoint of one Multipole leaf: one walk over the harmonics per point
  * ADDS this leaf's position VJP, A sigma (g_phi grad Phi - sigma H g_force),
  * into g_xyz [N,3] and accumulates the coefficient gradient into g_table as
