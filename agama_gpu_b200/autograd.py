@@ -26,6 +26,18 @@ from . import _lib
 from .potentials import prep_xyz
 
 
+def _one_walk(pot, t: float, want: set, precision) -> bool:
+    """Whether the fused adjoint gives exactly the gradients asked for at t: FP64 (the table
+    gradients are FP64 in either precision), and every expansion of the tree a Multipole with
+    a regular column structure whose node tensors are tracked."""
+    from . import potentials
+    if (precision or pot.precision or potentials._default_precision) != "fp64":
+        return False
+    exp = [c for c, _, _, _ in pot._leaves(float(t))
+           if c.kind in (_lib.KIND_MULTIPOLE, _lib.KIND_CYLSPLINE)]
+    return all(c.kind == _lib.KIND_MULTIPOLE and c._structure != 0 and id(c) in want for c in exp)
+
+
 class _PhiForce(torch.autograd.Function):
     @staticmethod
     def forward(ctx, xyz, pot, t, precision, tracked, *nodes):
@@ -40,11 +52,19 @@ class _PhiForce(torch.autograd.Function):
         (arr,) = ctx.saved_tensors
         pot, t = ctx.pot, ctx.t
         gx = None
+        node_grads = [None] * sum(len(p) for _, p in ctx.tracked)
+        nodes = any(ctx.needs_input_grad[5:])
+        want = {id(c) for c, _ in ctx.tracked}
+        if nodes and ctx.needs_input_grad[0] and _one_walk(pot, t, want, ctx.precision):
+            # positions and tables from one walk of each Multipole: 125 + 304 -> 236 us at
+            # 200k points, lmax 12, FP64
+            acc = {}
+            gx = pot._adjoint_vjp(arr, t, g_phi, g_force, acc, precision=ctx.precision)
+            node_grads = pot._node_param_grads(pot._table_grads_from_device(acc), ctx.tracked)
+            return (gx, None, None, None, None, *node_grads)
         if ctx.needs_input_grad[0]:
             gx = pot._vjp(arr, t, g_phi, g_force, precision=ctx.precision)
-        node_grads = [None] * sum(len(p) for _, p in ctx.tracked)
-        if any(ctx.needs_input_grad[5:]):
-            want = {id(c) for c, _ in ctx.tracked}
+        if nodes:
             acc = {}
             for comp, sigma, gamma, ampl in pot._leaves(float(t)):
                 if id(comp) not in want:

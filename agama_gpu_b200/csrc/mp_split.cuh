@@ -3,17 +3,16 @@
 // With one thread per point a call of a few thousand points leaves most of the GPU idle
 // while each thread walks every harmonic in turn: 1000 points are 32 warps on 148 SMs, each
 // with a chain of 289 steps at lmax 32.  Here a block takes a tile of at most 32 points
-// (lane = point) and its warps share the |m| groups, dealt out in snake order so that every
-// warp gets about the same number of (l, m) steps; all lanes of a warp walk the same (l, m),
+// (lane = point) and its warps share the |m| groups; all lanes of a warp walk the same (l, m),
 // so there is no divergence and the recurrence constants stay uniform.  A group's sums are
-// formed by the operations of mp_harmonics_reg; each warp adds its own groups up in FP64
-// and one warp adds the warps' sums and finishes the leaf (with Hessians the groups are kept
-// apart and added in their order).  Consecutive leaves take turns between two buffers and
+// formed by the operations of mp_harmonics_reg; the groups are added up slice by slice in
+// FP64 and one warp adds the slices' sums and finishes the leaf (with Hessians the groups are
+// kept apart and added in their order).  Consecutive leaves take turns between two buffers and
 // between finishing warps, so a leaf is finished while the next one is walked.
 #pragma once
 #include "multipole.cuh"
 
-// sums of a point that its warps add up
+// sums of a point that each slice adds up
 __host__ __device__ constexpr int split_sums(int mode) { return mode == AGB_MODE_POT ? 1 : 4; }
 // and, with Hessians, the values kept per |m| group: six of each trig column
 #define AGB_SPLIT_HESS_COLS 12
@@ -133,13 +132,18 @@ __device__ __forceinline__ void mp_each_sum(MPSums& t, F f)
     if (MODE == AGB_MODE_GRAD) { f(2, t.Th); f(3, t.Pos); }
 }
 
-// One warp's share of a leaf's groups: m = p S + w on even passes p, p S + S-1-w on odd ones.
-// The sums of its groups are added up in FP64 (tot); with Hessians, where the order of the
-// groups shows (see mp_combine_hess), each group's columns are kept in cols [m][value][point]
-// for mp_split_hess.
+// The |m| groups are dealt out to `slices` in snake order: slice v of V takes m = p V + v on
+// even passes p and p V + V-1-v on odd ones, which gives every slice about the same number of
+// (l, m) steps.  A warp takes the slices w, w + S, ...  The slices depend on lmax alone, so a
+// point's sums do not depend on the number of warps.
+__host__ __device__ constexpr int split_slices(int lmax) { return lmax / 2 + 1 < 16 ? lmax / 2 + 1 : 16; }
+
+// The sums over slice v's groups, added up in FP64 (tot); with Hessians, where the order of
+// the groups shows (see mp_combine_hess), each group's columns are kept in cols
+// [m][value][point] for mp_split_hess.
 template <int MODE, typename R, int PAR>
 __device__ __forceinline__ void mp_split_walk(const DevComp& c, int k, double s, double cth_d,
-                                              double sth_d, double cph, double sph, int w, int S,
+                                              double sth_d, double cph, double sph, int v, int V,
                                               MPSums& tot, R* cols, int T)
 {
     constexpr bool HESS = MODE == AGB_MODE_HESS;
@@ -148,8 +152,8 @@ __device__ __forceinline__ void mp_split_walk(const DevComp& c, int k, double s,
     const int lmax = c.lmax;
     double cm = 1.0, sm = 0.0, sinpow = 1.0, sinpow_m1 = 0.0;
     int at = 0;
-    for (int p = 0; p * S <= lmax; ++p) {
-        const int m = p * S + ((p & 1) ? S - 1 - w : w);
+    for (int p = 0; p * V <= lmax; ++p) {
+        const int m = p * V + ((p & 1) ? V - 1 - v : v);
         if (m > lmax) continue;
         for (; at < m; ++at) {
             if (!HESS) mp_rotate(cm, sm, cph, sph);

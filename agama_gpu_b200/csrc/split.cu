@@ -6,7 +6,7 @@
 // A few points per block, the harmonics split over its warps (mp_split.cuh): calls too small
 // to fill the GPU with one thread per point.  Block b evaluates the tile of a.chunk <= 32
 // points from b * a.chunk on.  Dynamic shared memory: two buffers of a.split_buf bytes with the
-// warps' sums [warp][sum][point] (Hessians: the groups' columns [m][value][point]), then every
+// slices' sums [slice][sum][point] (Hessians: the groups' columns [m][value][point]), then every
 // leaf's results [leaf][value][point].
 template <int MODE, typename R, bool DYN>
 __global__ void __launch_bounds__(split_threads(MODE), 1)
@@ -26,7 +26,7 @@ agb_split_kernel(const __grid_constant__ EvalArgs a)
     const int T = (int)a.chunk;
     const long long pos = (long long)blockIdx.x * T + lane;
     const bool live = lane < T && pos < a.n;
-    double* res = reinterpret_cast<double*>(split_smem + a.split_bufs * a.split_buf);
+    double* res = reinterpret_cast<double*>(split_smem + 2 * a.split_buf);
     double x = 0.0, y = 0.0, z = 0.0;
     if (live) {
         if (a.soa) {
@@ -44,6 +44,7 @@ agb_split_kernel(const __grid_constant__ EvalArgs a)
         const double ly = lf.sigma * y - lf.g1;
         const double lz = lf.sigma * z - lf.g2;
         const bool walked = c.kind == AGB_KIND_MULTIPOLE && c.structure != AGB_STRUCT_LIST;
+        const int V = split_slices(c.lmax);
         bool mine, grid = false;
         int k = 0;
         double s = 0.0, inv_r = 0.0, Rc = 0.0, cth = 1.0, sth = 0.0, cph = 1.0, sph = 0.0;
@@ -61,13 +62,15 @@ agb_split_kernel(const __grid_constant__ EvalArgs a)
                     sth = Rc * inv_r;
                     cph = (Rc > 1.0e-300) ? lx / Rc : 1.0;
                     sph = (Rc > 1.0e-300) ? ly / Rc : 0.0;
-                    MPSums t = {};
-                    if (c.structure == AGB_STRUCT_EVEN)
-                        mp_split_walk<CM, R, 2>(c, k, s, cth, sth, cph, sph, w, S, t, cols, T);
-                    else
-                        mp_split_walk<CM, R, 1>(c, k, s, cth, sth, cph, sph, w, S, t, cols, T);
-                    if (!HESS)
-                        mp_each_sum<CM>(t, [&](int q, double& v) { sums[(w * NS + q) * T] = v; });
+                    for (int v = w; v < V; v += S) {
+                        MPSums t = {};
+                        if (c.structure == AGB_STRUCT_EVEN)
+                            mp_split_walk<CM, R, 2>(c, k, s, cth, sth, cph, sph, v, V, t, cols, T);
+                        else
+                            mp_split_walk<CM, R, 1>(c, k, s, cth, sth, cph, sph, v, V, t, cols, T);
+                        if (!HESS)
+                            mp_each_sum<CM>(t, [&](int q, double& u) { sums[(v * NS + q) * T] = u; });
+                    }
                 }
             }
             __syncthreads();
@@ -91,8 +94,8 @@ agb_split_kernel(const __grid_constant__ EvalArgs a)
                 else
                     mp_split_hess<R, 1>(c.lmax, cth, sth, cph, sph, cols, T, t);
             } else {
-                for (int v = 0; v < S; ++v)
-                    mp_each_sum<CM>(t, [&](int q, double& x) { x += sums[(v * NS + q) * T]; });
+                for (int v = 0; v < V; ++v)
+                    mp_each_sum<CM>(t, [&](int q, double& u) { u += sums[(v * NS + q) * T]; });
             }
             mp_close<CM>(c, k, s, t, lx, ly, lz, inv_r, Rc, cth, sth, cph, sph, o);
         } else {
@@ -143,15 +146,14 @@ agb_split_kernel(const __grid_constant__ EvalArgs a)
 #define AGB_SPLIT_SMEM (220 * 1024)
 
 // Estimated time of an SM that evaluates `tiles` tiles with S warps each (S = 1: one thread
-// per point), `cap` tiles at a time: per wave of resident warps the walk's steps, each as long as the latency of one
-// step (lat) or as its warps keep the pipe busy, and the tile's finish, in units of one warp's
-// pipe time per step.
+// per point), `cap` tiles at a time: per wave of resident warps the steps of a warp, each as
+// long as the latency of one step (lat) or as the warps keep the pipe busy, and the tile's
+// finish, in units of one warp's pipe time per step.
 static long long split_cost(long long tiles, int S, long long cap, long long steps, int lat,
                             int finish)
 {
-    const long long per_warp = (steps + S - 1) / S;
     const long long full = tiles / cap, rest = tiles % cap;
-    auto wave = [&](long long n) { return per_warp * std::max<long long>(lat, n * S) + finish; };
+    auto wave = [&](long long n) { return steps * std::max<long long>(lat, n * S) + finish; };
     return full * wave(cap) + (rest ? wave(rest) : 0);
 }
 
@@ -160,7 +162,8 @@ static long long split_cost(long long tiles, int S, long long cap, long long ste
 //
 // T spreads the points over the SMs, at most 32 to a tile.  S comes from the estimate above:
 // an SM holds 16 warps at 128 registers (8 at 255, the Hessian modes), a step's latency is
-// about the pipe time of 11 warps (6), and finishing a leaf of a tile costs about 60 steps of one warp.
+// about the pipe time of 11 warps (6), and finishing a leaf of a tile costs about 60 steps of
+// one warp.
 // Measured (Multipole alone, FP64 force, one thread per point -> split): lmax 32 10k points
 // 119 -> 45 us (S = 5), 20k 119 -> 73 (S = 3), 40k 167 -> 138 (S = 3), 100k 331 -> 290
 // (S = 2), 300k 661 -> 768; lmax 16 40k 50 -> 46, 100k 96 -> 90; lmax 8 10k 15.5 -> 9.1,
@@ -174,58 +177,37 @@ static bool split_shape(EvalArgs& a, int& S, int& T, size_t& smem)
     if (a.out_flags & AGB_OUT_SHAPE_BITS) return false;        // the caller's launch shape
     const long long sms = num_sms();
     if (a.n > sms * 32 * 22) return false;
+    // the heaviest Multipole stands for the tree: device-time leaves, which may pick any of the
+    // components, and the same leaves given by the host get the same kernel and the same bits
     int lmax = 0;
-    long long steps = 0, one = 0;       // (l, |m|) pairs of the tree's walks
-    int walks = 0;
-    auto pairs = [](const DevComp& c) {
+    long long steps = 0;                // (l, |m|) pairs of its walk
+    for (const DevComp& c : a.comps) {
+        if (c.kind != AGB_KIND_MULTIPOLE || c.structure == AGB_STRUCT_LIST) continue;
         const long long h = c.lmax / 2 + 1, l1 = c.lmax + 1;
-        return c.structure == AGB_STRUCT_EVEN ? h * h : l1 * (l1 + 1) / 2;
-    };
-    auto split = [](const DevComp& c) {
-        return c.kind == AGB_KIND_MULTIPOLE && c.structure != AGB_STRUCT_LIST;
-    };
-    if (a.dleaves) {                    // device-time leaves may pick any component
-        for (const DevComp& c : a.comps)
-            if (split(c)) {
-                lmax = std::max(lmax, c.lmax);
-                steps = std::max(steps, pairs(c));
-            }
-        one = steps;
-        walks = a.n_leaves;
-    }
-    for (int L = 0; L < a.n_leaves && !a.dleaves; ++L) {
-        const DevComp& c = a.comps[a.leaves[L].comp];
-        if (!split(c)) continue;
         lmax = std::max(lmax, c.lmax);
-        ++walks;
-        steps += pairs(c);
-        // one thread per point walks two bracketing snapshots at once (mixed precision)
-        one += L > 0 && a.leaves[L - 1].pad == 1 ? pairs(c) * 6 / 10 : pairs(c);
+        steps = std::max(steps, c.structure == AGB_STRUCT_EVEN ? h * h : l1 * (l1 + 1) / 2);
     }
     if (lmax < 2) return false;
     T = (int)std::min<long long>(32, (a.n + sms - 1) / sms);
     const long long tiles = ((a.n + T - 1) / T + sms - 1) / sms;     // of an SM
-    auto bytes = [&](int s) {           // of dynamic shared memory; one buffer serves one walk
-        a.split_buf = T * (CM == AGB_MODE_HESS ? (lmax + 1) * AGB_SPLIT_HESS_COLS * (int)sizeof(R)
-                                               : s * split_sums(CM) * (int)sizeof(double));
-        a.split_buf = (a.split_buf + 15) & ~15;
-        return (walks > 1 ? 2 : 1) * (size_t)a.split_buf + sizeof(double) * T * (size_t)a.n_leaves * split_out(CM);
-    };
+    const int V = split_slices(lmax);
+    a.split_buf = T * (CM == AGB_MODE_HESS ? (lmax + 1) * AGB_SPLIT_HESS_COLS * (int)sizeof(R)
+                                           : V * split_sums(CM) * (int)sizeof(double));
+    a.split_buf = (a.split_buf + 15) & ~15;
+    // tiles that fit an SM's shared memory, with the results of eight leaves
+    const int fit = AGB_SPLIT_SMEM / (2 * a.split_buf + 8 * split_out(CM) * T * (int)sizeof(double));
     const int lat = warps == 16 ? 11 : 6;
-    long long best = split_cost(tiles, S = 1, warps, one, lat, 0);
-    for (int s = 2; s <= std::min(warps, lmax / 2 + 1); ++s) {
-        const long long cap = std::min<long long>(warps / s, AGB_SPLIT_SMEM / bytes(s));
-        if (cap < 1) continue;
-        const long long t = split_cost(tiles, s, cap, steps, lat, 60 * walks);
+    long long best = split_cost(tiles, S = 1, warps, steps, lat, 0);
+    for (int s = 2; s <= std::min(warps, V); ++s) {
+        const int cap = std::max(1, std::min(warps / s, fit));
+        const long long t = split_cost(tiles, s, cap, steps * ((V + s - 1) / s) / V, lat, 60);
         if (t < best) {
             best = t;
             S = s;
         }
     }
-    if (S < 2) return false;
-    smem = bytes(S);
-    a.split_bufs = walks > 1 ? 2 : 1;
-    return true;
+    smem = 2 * (size_t)a.split_buf + sizeof(double) * T * (size_t)a.n_leaves * split_out(CM);
+    return S >= 2 && smem <= AGB_SPLIT_SMEM;
 }
 
 template <int MODE, typename R, bool DYN>
