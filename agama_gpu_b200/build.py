@@ -27,7 +27,7 @@ STAMP = PKG / ".libagb.stamp"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC",
               "--expt-relaxed-constexpr", "-Xptxas", "-v"]
-SOURCES = ["eval.cu", "split.cu", "nodes.cu", "peak.cu"]
+SOURCES = ["eval.cu", "split.cu", "cyl.cu", "nodes.cu", "peak.cu"]
 
 
 def _nvcc() -> str:

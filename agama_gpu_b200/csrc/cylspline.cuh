@@ -63,6 +63,63 @@ __device__ __forceinline__ void cs_bicubic(const T v[16], T tR, T TR, T tTR, T h
         cs_hermite<T>(tR, TR, tTR, hR, d2F[0], d2F[1], d2F[2], d2F[3], &vzz, nullptr, nullptr);
 }
 
+// FP64: the same interpolation as weights of the 16 node values, formed once per point and
+// axis (Hermite basis functions, their first and second derivatives), so that a harmonic
+// costs 54 operations and no division (the form above has six divisions by the cell's
+// widths).  The values enter as one end's and the difference to the other's.
+struct CSAxis {
+    double H, S0, S1;              // of the difference of the end values, of the end slopes
+    double dH, dS0, dS1;           // first derivatives
+    double eH, eS0, eS1;           // second derivatives
+};
+
+template <bool DO_G, bool DO_H>
+__device__ __forceinline__ CSAxis cs_axis(double t, double T, double h)
+{
+    CSAxis w;
+    const double tT = t * T;
+    w.H = t * t * (1.0 + 2.0 * T);
+    w.S0 = tT * T * h;
+    w.S1 = -tT * t * h;
+    const double ih = (DO_G || DO_H) ? 1.0 / h : 0.0;
+    w.dH = 6.0 * tT * ih;
+    w.dS0 = T * (T - 2.0 * t);
+    w.dS1 = t * (t - 2.0 * T);
+    w.eH = 6.0 * (T - t) * ih * ih;
+    w.eS0 = (2.0 * t - 4.0 * T) * ih;
+    w.eS1 = (4.0 * t - 2.0 * T) * ih;
+    return w;
+}
+
+template <bool DO_G, bool DO_H>
+__device__ __forceinline__ void cs_bicubic_w(const double v[16], const CSAxis& R, const CSAxis& z,
+                                             double& val, double& vR, double& vRR, double& vz,
+                                             double& vRz, double& vzz)
+{
+    double F[4], dF[4], d2F[4];
+    #pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const double a = v[2 * q], b = v[2 * q + 1], sa = v[8 + 2 * q], sb = v[9 + 2 * q];
+        const double d = b - a;
+        F[q] = fma(z.H, d, fma(z.S0, sa, fma(z.S1, sb, a)));
+        if (DO_G) dF[q] = fma(z.dH, d, fma(z.dS0, sa, z.dS1 * sb));
+        if (DO_H) d2F[q] = fma(z.eH, d, fma(z.eS0, sa, z.eS1 * sb));
+    }
+    auto value = [&](const double f[4]) {
+        return fma(R.H, f[1] - f[0], fma(R.S0, f[2], fma(R.S1, f[3], f[0])));
+    };
+    auto slope = [&](const double f[4]) {
+        return fma(R.dH, f[1] - f[0], fma(R.dS0, f[2], R.dS1 * f[3]));
+    };
+    val = value(F);
+    if (DO_G) { vR = slope(F); vz = value(dF); }
+    if (DO_H) {
+        vRR = fma(R.eH, F[1] - F[0], fma(R.eS0, F[2], R.eS1 * F[3]));
+        vRz = slope(dF);
+        vzz = value(d2F);
+    }
+}
+
 // Outer PowerLaw multipole (W_outer, r0) evaluated with the reference's
 // simplifications (no theta term in the gradient, monopole-only Hessian) and
 // its angular basis (see legendre.outer_asymptote_basis on the host side).
@@ -73,9 +130,9 @@ __device__ void cs_outer(const DevComp& c, double x, double y, double z, PointOu
     const double r0 = c.p[1];
     const int lmax = c.lmax;
     const int mmax = (int)c.p[2];
-    const double R2 = x * x + y * y;
+    const double R2 = fma(x, x, __dmul_rn(y, y));
     const double R = sqrt(R2);
-    const double r = sqrt(R2 + z * z);
+    const double r = sqrt(fma(z, z, R2));
     const double rinv = 1.0 / r;
     const double ct = z * rinv, st = R * rinv;
     const double cph = (R > 0.0) ? x / R : 1.0;
@@ -100,27 +157,30 @@ __device__ void cs_outer(const DevComp& c, double x, double y, double z, PointOu
                 Pl = p * AGB_NORM[m * AGB_LEG_N + l];
                 pw *= rr;
             } else {
-                const double nw = (ct * (double)(2 * l - 1) * p - (double)(l + m - 1) * p2) / (double)(l - m);
+                const double nw = fma(__dmul_rn(ct, (double)(2 * l - 1)), p, -__dmul_rn((double)(l + m - 1), p2)) / (double)(l - m);
                 p2 = p1; p1 = p; p = nw;
                 Pl = nw * AGB_NORM[m * AGB_LEG_N + l];
                 pw *= rr;
             }
             const double Yb = Pl * MUL;
+            // sums with their roundings spelled out: the kernels of both precisions agree here
+            // to the last bit
             if (m == 0) {
-                const double w = __ldg(W + l * (l + 1));
-                phi += w * pw * Yb;
-                dr += w * (double)(-(l + 1)) * rinv * pw * Yb;
+                const double t = __dmul_rn(__dmul_rn(__ldg(W + l * (l + 1)), pw), Yb);
+                phi = __dadd_rn(phi, t);
+                dr = fma(__dmul_rn((double)(-(l + 1)), rinv), t, dr);
             } else {
                 const double wc = __ldg(W + l * (l + 1) + m);
                 const double ws = __ldg(W + l * (l + 1) - m);
-                const double contrib = pw * Yb * (wc * cm + ws * sm);
-                phi += contrib;
-                dr += (double)(-(l + 1)) * rinv * contrib;
-                dphi += pw * Yb * (wc * (-(double)m * sm) + ws * ((double)m * cm));
+                const double f = __dmul_rn(pw, Yb);
+                const double t = __dmul_rn(f, fma(wc, cm, __dmul_rn(ws, sm)));
+                phi = __dadd_rn(phi, t);
+                dr = fma(__dmul_rn((double)(-(l + 1)), rinv), t, dr);
+                dphi = fma(__dmul_rn(f, (double)m), fma(ws, cm, -__dmul_rn(wc, sm)), dphi);
             }
         }
-        const double t = cm * cph - sm * sph;
-        sm = sm * cph + cm * sph;
+        const double t = fma(cm, cph, -__dmul_rn(sm, sph));
+        sm = fma(sm, cph, __dmul_rn(cm, sph));
         cm = t;
         sinpow *= st;
     }
@@ -128,8 +188,8 @@ __device__ void cs_outer(const DevComp& c, double x, double y, double z, PointOu
     if (MODE == AGB_MODE_GRAD || MODE == AGB_MODE_HESS) {
         const double dphx = (R > 1e-30) ? -y / R2 : 0.0;
         const double dphy = (R > 1e-30) ? x / R2 : 0.0;
-        o.g[0] = dr * (x * rinv) + dphi * dphx;
-        o.g[1] = dr * (y * rinv) + dphi * dphy;
+        o.g[0] = fma(dr, x * rinv, __dmul_rn(dphi, dphx));
+        o.g[1] = fma(dr, y * rinv, __dmul_rn(dphi, dphy));
         o.g[2] = dr * (z * rinv);
     }
     if (MODE == AGB_MODE_HESS || MODE == AGB_MODE_DENS) {
@@ -191,8 +251,208 @@ __device__ __forceinline__ double cs_load32(const DevComp& c, int h, int iR, int
     return __hiloint2double(__float_as_int(q0.y), __float_as_int(q0.x));
 }
 
-template <int MODE, bool EXACT = false, typename RT = double>
-__device__ __forceinline__ void cylspline_point(const DevComp& c, double px, double py,
+// A point's cylindrical and scaled coordinates and its cell.
+struct CSPlace {
+    double R2, R, lR, lz;
+    int iR, iz;
+    double hR, hz, tR, tz;
+    bool R_at_hi, z_at_hi;
+};
+
+// false beyond the (lR, lz) grid (cs_outer gives the result there)
+__device__ __forceinline__ bool cs_place(const DevComp& c, double px, double py, double pz, CSPlace& q)
+{
+    const double Rs = c.p[0];
+    const double* __restrict__ lRg = c.grid_a;
+    const double* __restrict__ lzg = c.grid_b;
+    const int nR = c.n_int, nz = c.nz;
+    q.R2 = px * px + py * py;
+    q.R = sqrt(q.R2);
+    q.lR = asinh(q.R / Rs);
+    q.lz = asinh(pz / Rs);
+    if (q.lR < __ldg(lRg) || q.lR > __ldg(lRg + nR - 1) || q.lz < __ldg(lzg) || q.lz > __ldg(lzg + nz - 1))
+        return false;
+    q.iR = cs_cell(q.lR, lRg, nR);
+    q.iz = cs_cell(q.lz, lzg, nz);
+    const double lR_lo = __ldg(lRg + q.iR), lR_hi = __ldg(lRg + q.iR + 1);
+    const double lz_lo = __ldg(lzg + q.iz), lz_hi = __ldg(lzg + q.iz + 1);
+    q.hR = lR_hi - lR_lo;
+    q.hz = lz_hi - lz_lo;
+    q.tR = (q.lR - lR_lo) / q.hR;
+    q.tz = (q.lz - lz_lo) / q.hz;
+    q.R_at_hi = q.lR == lR_hi;
+    q.z_at_hi = q.lz == lz_hi;
+    return true;
+}
+
+// The Fourier sums of a point: of the harmonics beyond m = 0 and, under log-scaling, the m = 0
+// term's spline.
+struct CSSums {
+    double S, S_R, S_z, S_RR, S_Rz, S_zz, S_p, S_pp, S_Rp, S_zp;
+    double f0, f0R, f0z, f0RR, f0Rz, f0zz;
+};
+
+// One cell's records straight from global memory.
+struct CSGlobal {
+    const DevComp& c;
+    int iR, iz;
+    __device__ __forceinline__ void rec64(int h, double v[16]) const { cs_load(c, h, iR, iz, v); }
+};
+
+// FP64.  load: the records of harmonic 0, 1, ... of the point's cell
+template <int MODE, typename Loader>
+__device__ __forceinline__ void cs_harmonics(const DevComp& c, const CSPlace& q, double cph,
+                                             double sph, const Loader& load, CSSums& s)
+{
+    constexpr bool DO_G = MODE != AGB_MODE_POT;
+    constexpr bool DO_H = MODE == AGB_MODE_HESS || MODE == AGB_MODE_DENS;
+    const int ls = c.log_scaling;
+    const CSAxis wR = cs_axis<DO_G, DO_H>(q.tR, 1.0 - q.tR, q.hR);
+    const CSAxis wz = cs_axis<DO_G, DO_H>(q.tz, 1.0 - q.tz, q.hz);
+    s = {};
+    s.S = ls ? 1.0 : 0.0;
+    int cur = 0;
+    double cm = 1.0, sm = 0.0;
+    for (int h = 0; h < c.n_lm; ++h) {
+        const int m = __ldg(c.lm + h);
+        double val, vR = 0.0, vRR = 0.0, vz = 0.0, vRz = 0.0, vzz = 0.0;
+        double v[16];
+        load.rec64(h, v);
+        const double off = q.R_at_hi ? (q.z_at_hi ? v[3] : v[2]) : (q.z_at_hi ? v[1] : v[0]);
+        v[0] -= off; v[1] -= off; v[2] -= off; v[3] -= off;
+        cs_bicubic_w<DO_G, DO_H>(v, wR, wz, val, vR, vRR, vz, vRz, vzz);
+        val += off;
+
+        double T = 1.0, dT = 0.0, d2T = 0.0;
+        if (m != 0) {
+            const int am = m < 0 ? -m : m;
+            if (am < cur) { cur = 0; cm = 1.0; sm = 0.0; }
+            for (; cur < am; ++cur) {
+                const double t = cm * cph - sm * sph;
+                sm = sm * cph + cm * sph;
+                cm = t;
+            }
+            if (m > 0) { T = cm; dT = -(double)am * sm; d2T = -(double)(am * am) * cm; }
+            else       { T = sm; dT = (double)am * cm; d2T = -(double)(am * am) * sm; }
+        }
+        if (m == 0) {
+            s.f0 = val; s.f0R = vR; s.f0z = vz; s.f0RR = vRR; s.f0Rz = vRz; s.f0zz = vzz;
+            if (!ls) {
+                s.S += val; s.S_R += vR; s.S_z += vz;
+                if (DO_H) { s.S_RR += vRR; s.S_Rz += vRz; s.S_zz += vzz; }
+            }
+        } else {
+            s.S += val * T; s.S_R += vR * T; s.S_z += vz * T; s.S_p += val * dT;
+            if (DO_H) {
+                s.S_RR += vRR * T; s.S_Rz += vRz * T; s.S_zz += vzz * T;
+                s.S_Rp += vR * dT; s.S_zp += vz * dT; s.S_pp += val * d2T;
+            }
+        }
+    }
+}
+
+// Un-scaling and the conversion to Cartesian derivatives of a point inside the grid.
+template <int MODE, bool EXACT>
+__device__ __forceinline__ void cs_close(const DevComp& c, double px, double py, double pz,
+                                         const CSPlace& q, const CSSums& s, PointOut& o)
+{
+    constexpr bool DO_G = MODE != AGB_MODE_POT;
+    constexpr bool DO_H = MODE == AGB_MODE_HESS || MODE == AGB_MODE_DENS;
+    const double Rs = c.p[0], R2 = q.R2, R = q.R;
+    const int ls = c.log_scaling;
+    const double dlRdR = 1.0 / sqrt(R2 + Rs * Rs);
+    const double dlzdz = 1.0 / sqrt(pz * pz + Rs * Rs);
+    const double d2lRdR2 = -R * dlRdR * dlRdR * dlRdR;
+    const double d2lzdz2 = -pz * dlzdz * dlzdz * dlzdz;
+    double P, PR = 0.0, Pz = 0.0, Pp = s.S_p, PRR = 0.0, PRz = 0.0, Pzz = 0.0;
+    double PRp = 0.0, Pzp = 0.0, Ppp = s.S_pp;
+    if (ls) {
+        const double P0 = -exp(s.f0);
+        const double P0R = P0 * s.f0R, P0z = P0 * s.f0z;
+        P = P0 * s.S;
+        if (DO_G) { PR = P0 * s.S_R + P0R * s.S; Pz = P0 * s.S_z + P0z * s.S; Pp = P0 * s.S_p; }
+        if (DO_H) {
+            const double P0RR = P0 * (s.f0RR + s.f0R * s.f0R);
+            const double P0zz = P0 * (s.f0zz + s.f0z * s.f0z);
+            const double P0Rz = P0 * (s.f0Rz + s.f0R * s.f0z);
+            PRR = P0 * s.S_RR + 2.0 * P0R * s.S_R + P0RR * s.S;
+            Pzz = P0 * s.S_zz + 2.0 * P0z * s.S_z + P0zz * s.S;
+            PRz = P0 * s.S_Rz + P0R * s.S_z + P0z * s.S_R + P0Rz * s.S;
+            PRp = P0 * s.S_Rp + P0R * s.S_p;
+            Pzp = P0 * s.S_zp + P0z * s.S_p;
+            Ppp = P0 * s.S_pp;
+        }
+    } else {
+        P = s.S; PR = s.S_R; Pz = s.S_z;
+        if (DO_H) { PRR = s.S_RR; Pzz = s.S_zz; PRz = s.S_Rz; PRp = s.S_Rp; Pzp = s.S_zp; }
+    }
+    o.phi = P;
+    if (!DO_G) return;
+
+    const double dPdR = PR * dlRdR;
+    const double dPdz = Pz * dlzdz;
+    double gx = 0.0, gy = 0.0;
+    if (R > 1e-30) {
+        const double Ri = 1.0 / R, R2i = Ri * Ri;
+        gx = dPdR * (px * Ri) - Pp * (py * R2i);
+        gy = dPdR * (py * Ri) + Pp * (px * R2i);
+    }
+    o.g[0] = gx; o.g[1] = gy; o.g[2] = dPdz;
+    if (!DO_H) return;
+
+    const double H_RR = PRR * (dlRdR * dlRdR) + PR * d2lRdR2;
+    const double H_zz = Pzz * (dlzdz * dlzdz) + Pz * d2lzdz2;
+    const double H_Rz = PRz * dlRdR * dlzdz;
+    const double H_pp = Ppp;
+    const double H_Rp = PRp * dlRdR;
+    const double H_zp = Pzp * dlzdz;
+    if (R > 1e-30) {
+        const double Ri = 1.0 / R, R2i = Ri * Ri, R3i = R2i * Ri;
+        const double x = px, y = py, x2 = x * x, y2 = y * y, xy = x * y;
+        o.h[0] = H_RR * x2 * R2i - 2.0 * H_Rp * xy * R3i + H_pp * y2 * R2i * R2i + dPdR * y2 * R3i;
+        o.h[1] = H_RR * y2 * R2i + 2.0 * H_Rp * xy * R3i + H_pp * x2 * R2i * R2i + dPdR * x2 * R3i;
+        o.h[2] = H_zz;
+        o.h[3] = H_RR * xy * R2i + H_Rp * (x2 - y2) * R3i - H_pp * xy * R2i * R2i - dPdR * xy * R3i;
+        o.h[4] = H_Rz * (y * Ri) + H_zp * (x * R2i);
+        o.h[5] = H_Rz * (x * Ri) - H_zp * (y * R2i);
+        if (EXACT) {
+            const double R4i = R2i * R2i;
+            o.h[0] += 2.0 * Pp * xy * R4i;
+            o.h[1] -= 2.0 * Pp * xy * R4i;
+            o.h[3] += Pp * (y2 - x2) * R4i;
+        }
+    } else {
+        o.h[0] = H_RR; o.h[1] = H_RR; o.h[2] = H_zz;
+        o.h[3] = 0.0; o.h[4] = 0.0; o.h[5] = 0.0;
+    }
+    // the reference's CylSpline density is -(Hxx+Hyy+Hzz)/(4 pi G)
+    // (gpu_potential.py:1389-1395); kept for parity
+    if (MODE == AGB_MODE_DENS) o.rho = -(o.h[0] + o.h[1] + o.h[2]) * AGB_INV_4PIG;
+}
+
+template <int MODE, bool EXACT>
+__device__ __forceinline__ void cs_point(const DevComp& c, double px, double py,
+                                                double pz, PointOut& o)
+{
+    CSPlace q;
+    if (!cs_place(c, px, py, pz, q)) {
+        cs_outer<MODE>(c, px, py, pz, o);
+        if (MODE == AGB_MODE_DENS) o.rho = -(o.h[0] + o.h[1] + o.h[2]) * AGB_INV_4PIG;
+        return;
+    }
+    const double cph = (q.R > 0.0) ? px / q.R : 1.0;
+    const double sph = (q.R > 0.0) ? py / q.R : 0.0;
+    CSSums s;
+    cs_harmonics<MODE>(c, q, cph, sph, CSGlobal{c, q.iR, q.iz}, s);
+    cs_close<MODE, EXACT>(c, px, py, pz, q, s, o);
+}
+
+// Mixed precision, in one body of its own: built from the pieces above the FP32 Multipole walk
+// of the same kernels spills more (4M-point composite 4.18 -> 4.79 ms; 4.60 ms with the
+// CylSpline in a function that is called), and a disk's points gain nothing from loads shared
+// by a warp (force at 1M points 183 -> 194 us: bound by the FP32 Hermite's divisions).
+template <int MODE, bool EXACT, typename RT>
+__device__ __forceinline__ void cs_point_mixed(const DevComp& c, double px, double py,
                                                 double pz, PointOut& o)
 {
     constexpr bool F32 = std::is_same<RT, float>::value;   // mixed precision
@@ -349,4 +609,14 @@ __device__ __forceinline__ void cylspline_point(const DevComp& c, double px, dou
     // the reference's CylSpline density is -(Hxx+Hyy+Hzz)/(4 pi G)
     // (gpu_potential.py:1389-1395); kept for parity
     if (MODE == AGB_MODE_DENS) o.rho = -(o.h[0] + o.h[1] + o.h[2]) * AGB_INV_4PIG;
+}
+
+template <int MODE, bool EXACT = false, typename RT = double>
+__device__ __forceinline__ void cylspline_point(const DevComp& c, double px, double py,
+                                                double pz, PointOut& o)
+{
+    if constexpr (std::is_same<RT, float>::value)
+        cs_point_mixed<MODE, EXACT, RT>(c, px, py, pz, o);
+    else
+        cs_point<MODE, EXACT>(c, px, py, pz, o);
 }

@@ -324,6 +324,7 @@ static int launch_eval_mode(int mode, int precision, EvalArgs& a, cudaStream_t s
 {
     const bool mixed = precision == AGB_PREC_MIXED;
     if (agb_launch_split(mode, mixed, a, st)) return check_launch("agb_split_kernel");
+    if (agb_launch_cyl(mode, mixed, a, st)) return check_launch("agb_cyl_kernel");
     if (a.dleaves) {        // leaves computed on the device (agb_eval_timed)
         switch (mode) {
         case AGB_MODE_POT:  mixed ? launch_eval<AGB_MODE_POT, float, false, true>(a, st)  : launch_eval<AGB_MODE_POT, double, false, true>(a, st); break;

@@ -58,3 +58,6 @@ int agb_check_launch(const char* what);
 // split.cu: launches the split kernel (a few points per block, the harmonics shared by its
 // warps) where that is the better shape for this call; false where it is not
 bool agb_launch_split(int mode, bool mixed, EvalArgs& a, cudaStream_t st);
+
+// cyl.cu: the same for trees whose expansions are CylSplines
+bool agb_launch_cyl(int mode, bool mixed, EvalArgs& a, cudaStream_t st);

@@ -163,7 +163,7 @@ static long long split_cost(long long tiles, int S, long long cap, long long ste
 // T spreads the points over the SMs, at most 32 to a tile.  S comes from the estimate above:
 // an SM holds 16 warps at 128 registers (8 at 255, the Hessian modes), a step's latency is
 // about the pipe time of 11 warps (6), and finishing a leaf of a tile costs about 60 steps of
-// one warp.
+// one warp (twice that with Hessians).
 // Measured (Multipole alone, FP64 force, one thread per point -> split): lmax 32 10k points
 // 119 -> 45 us (S = 5), 20k 119 -> 73 (S = 3), 40k 167 -> 138 (S = 3), 100k 331 -> 290
 // (S = 2), 300k 661 -> 768; lmax 16 40k 50 -> 46, 100k 96 -> 90; lmax 8 10k 15.5 -> 9.1,
@@ -200,7 +200,8 @@ static bool split_shape(EvalArgs& a, int& S, int& T, size_t& smem)
     long long best = split_cost(tiles, S = 1, warps, steps, lat, 0);
     for (int s = 2; s <= std::min(warps, V); ++s) {
         const int cap = std::max(1, std::min(warps / s, fit));
-        const long long t = split_cost(tiles, s, cap, steps * ((V + s - 1) / s) / V, lat, 60);
+        const long long t = split_cost(tiles, s, cap, steps * ((V + s - 1) / s) / V, lat,
+                                       CM == AGB_MODE_HESS ? 120 : 60);
         if (t < best) {
             best = t;
             S = s;
