@@ -539,10 +539,9 @@ __device__ __forceinline__ void mp_adj_walk(const DevComp& c, int kw, R s, doubl
 {
     constexpr int MODE = AGB_MODE_HESS;
     const bool near_pole = sth_d < 1.0e-10;
-    R sp[6], dw[6], ew[6];
+    R sp[6], dw[6];
     sp[0] = R(1); sp[1] = s; sp[2] = s * s; sp[3] = sp[2] * s; sp[4] = sp[2] * sp[2]; sp[5] = sp[4] * s;
     dw[0] = R(0); dw[1] = R(1); dw[2] = R(2) * s; dw[3] = R(3) * sp[2]; dw[4] = R(4) * sp[3]; dw[5] = R(5) * sp[4];
-    ew[0] = R(0); ew[1] = R(0); ew[2] = R(2); ew[3] = R(6) * s; ew[4] = R(12) * sp[2]; ew[5] = R(20) * sp[3];
     const R cth = (R)cth_d, sth = (R)sth_d;
     const R c2 = (R)(cth_d * cth_d), w2 = (R)(-2.0 * cth_d * sth_d);   // two-step walk
     const R inv_sth = near_pole ? R(0) : (R)(1.0 / sth_d);
@@ -598,12 +597,12 @@ __device__ __forceinline__ void mp_adj_walk(const DevComp& c, int kw, R s, doubl
             R a[6], b[6];
             if (F32 && m > 0) MPPtr<R>::load_cs(rec, a, b);
             else MPPtr<R>::load(rec, a);
-            mp_col_acc<MODE, R>(gc, a, sp, dw, ew, Pc, dPc, ll1);
+            mp_col_acc<MODE, R>(gc, a, sp, Pc, dPc, ll1);
             adj_put<R, EMIT>(T, gbase, col++, sp, dw, fma(Tc, base, dTc * Pq), P2 * Pc * Tc, lane,
                              active);
             if (m > 0) {
                 if (!F32) MPPtr<R>::load(rec + MPPtr<R>::REC, b);
-                mp_col_acc<MODE, R>(gs, b, sp, dw, ew, Pc, dPc, ll1);
+                mp_col_acc<MODE, R>(gs, b, sp, Pc, dPc, ll1);
                 adj_put<R, EMIT>(T, gbase, col++, sp, dw, fma(Ts, base, dTs * Pq), P2 * Pc * Ts, lane,
                            active);
             }

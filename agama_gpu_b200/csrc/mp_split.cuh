@@ -48,10 +48,8 @@ __device__ __forceinline__ void mp_group(const R* rec, int m, int lmax, R s, dou
 {
     constexpr bool NEED_ANG = MODE == AGB_MODE_GRAD || MODE == AGB_MODE_HESS;
     const bool near_pole = sth_d < 1.0e-10;
-    R sp[6], dw[6], ew[6];
+    R sp[6];
     sp[0] = R(1); sp[1] = s; sp[2] = s * s; sp[3] = sp[2] * s; sp[4] = sp[2] * sp[2]; sp[5] = sp[4] * s;
-    dw[0] = R(0); dw[1] = R(1); dw[2] = R(2) * s; dw[3] = R(3) * sp[2]; dw[4] = R(4) * sp[3]; dw[5] = R(5) * sp[4];
-    ew[0] = R(0); ew[1] = R(0); ew[2] = R(2); ew[3] = R(6) * s; ew[4] = R(12) * sp[2]; ew[5] = R(20) * sp[3];
     const R cth = (R)cth_d, sth = (R)sth_d;
     const R c2 = (R)(cth_d * cth_d), w2 = (R)(-2.0 * cth_d * sth_d);
     int l0 = (PAR == 2) ? (m + (m & 1)) : m;
@@ -81,8 +79,8 @@ __device__ __forceinline__ void mp_group(const R* rec, int m, int lmax, R s, dou
         else MPPtr<R>::load(rec, ac);
         rec += has_sin ? 2 * MPPtr<R>::REC : MPPtr<R>::REC;
         const R ll1 = R(L * (L + 1));
-        mp_col_acc<MODE, R>(gc, ac, sp, dw, ew, Pc, dPc, ll1);
-        if (has_sin) mp_col_acc<MODE, R>(gs, as, sp, dw, ew, Pc, dPc, ll1);
+        mp_col_acc<MODE, R>(gc, ac, sp, Pc, dPc, ll1);
+        if (has_sin) mp_col_acc<MODE, R>(gs, as, sp, Pc, dPc, ll1);
     };
     const int ts = m * AGB_SKIP_N;
     auto skip2 = [&](int L) {

@@ -287,19 +287,27 @@ template <typename R> struct MPCol {         // per-group sums of one trig colum
 //   Y/sin         = Y inv_sth + q1 dY              (q1: the m=1 pole rule)
 //   d2Y/dtheta2   = np1 (-cot dY - (l(l+1) - m^2/sin^2) Y)
 // (the Legendre equation) have coefficients that do not depend on l.
+// C, C' and C''/2 in one Horner pass (5 + 4 + 3 multiply-adds against 5 + 5 + 5 for separate
+// sums); the C''/2 sum is doubled once per group in mp_col_finish.  Measured in FP64 against two
+// short chains per sum: densities 487 -> 420 us (500k points, lmax 20, every l), the 1M-point
+// lmax-32 tree's forces 1957 -> 1877, Hessians at lmax 16 232 -> 220 (300k points).  The potential
+// alone has one sum: 470 us either way, two chains.
+template <int MODE, typename R>
+__host__ __device__ constexpr bool mp_joint()
+{
+    return std::is_same<R, float>::value || MODE != AGB_MODE_POT;
+}
+
 template <int MODE, typename R>
 __device__ __forceinline__ void mp_col_acc(MPCol<R>& g, const R a[6], const R sp[6],
-                                           const R dw[6], const R ew[6], R Y, R dY, R ll1)
+                                           R Y, R dY, R ll1)
 {
     constexpr bool NEED_B = MODE != AGB_MODE_POT;
     constexpr bool NEED_D = MODE == AGB_MODE_HESS || MODE == AGB_MODE_DENS;
     constexpr bool NEED_ANG = MODE == AGB_MODE_GRAD || MODE == AGB_MODE_HESS;
-    // C = sum a_j s^j.  FP32: one Horner pass carries C, C' and C''/2 together
-    // (5 + 4 + 3 FMAs against 5 + 5 + 5 for separate sums); the C''/2 sum is doubled
-    // once per group in mp_col_finish.  FP64: two short chains per sum, where the
-    // longer dependent DFMA chain costs more than it saves
+    // C = sum a_j s^j
     R C, dC = R(0), d2C = R(0);
-    if (std::is_same<R, float>::value) {
+    if (mp_joint<MODE, R>()) {
         const R x = sp[1];
         R p = fma(a[5], x, a[4]), d = a[5], e = a[5];
         d = fma(d, x, p); p = fma(p, x, a[3]);
@@ -314,8 +322,6 @@ __device__ __forceinline__ void mp_col_acc(MPCol<R>& g, const R a[6], const R sp
         d2C = e;
     } else {
         C = fma(a[2], sp[2], fma(a[1], sp[1], a[0])) + fma(a[5], sp[5], fma(a[4], sp[4], a[3] * sp[3]));
-        if (NEED_B) dC = fma(a[2], dw[2], a[1]) + fma(a[5], dw[5], fma(a[4], dw[4], a[3] * dw[3]));
-        if (NEED_D) d2C = fma(a[3], ew[3], R(2) * a[2]) + fma(a[5], ew[5], a[4] * ew[4]);
     }
     g.V = fma(C, Y, g.V);
     if (NEED_B) {
@@ -333,8 +339,8 @@ __device__ __forceinline__ void mp_col_finish(MPCol<R>& g, R inv_sth, R q1, R np
 {
     if (MODE == AGB_MODE_GRAD || MODE == AGB_MODE_HESS) g.VP = fma(g.V, inv_sth, q1 * g.VT);
     if (MODE == AGB_MODE_HESS) g.VTT = np1 * (fma(-cot, g.VT, m2 * g.V) - g.L);
-    if ((MODE == AGB_MODE_HESS || MODE == AGB_MODE_DENS) && std::is_same<R, float>::value)
-        g.VRR *= R(2);                                          // the FP32 walk sums C''/2
+    if ((MODE == AGB_MODE_HESS || MODE == AGB_MODE_DENS) && mp_joint<MODE, R>())
+        g.VRR *= R(2);                                          // the joint pass sums C''/2
 }
 
 // One |m| group's sums combined with cos/sin(m phi), and the rotation to the next m, with
@@ -381,10 +387,8 @@ __device__ __forceinline__ void mp_harmonics_reg(const DevComp& c, int k, double
     constexpr bool NEED_ANG = MODE == AGB_MODE_GRAD || MODE == AGB_MODE_HESS;
     const bool near_pole = sth_d < 1.0e-10;
     const R s = (R)s_d;
-    R sp[6], dw[6], ew[6];
+    R sp[6];
     sp[0] = R(1); sp[1] = s; sp[2] = s * s; sp[3] = sp[2] * s; sp[4] = sp[2] * sp[2]; sp[5] = sp[4] * s;
-    dw[0] = R(0); dw[1] = R(1); dw[2] = R(2) * s; dw[3] = R(3) * sp[2]; dw[4] = R(4) * sp[3]; dw[5] = R(5) * sp[4];
-    ew[0] = R(0); ew[1] = R(0); ew[2] = R(2); ew[3] = R(6) * s; ew[4] = R(12) * sp[2]; ew[5] = R(20) * sp[3];
     const R cth = (R)cth_d, sth = (R)sth_d;
     const R c2 = (R)(cth_d * cth_d), w2 = (R)(-2.0 * cth_d * sth_d);   // two-step walk
     const R inv_sth = near_pole ? R(0) : (R)(1.0 / sth_d);
@@ -441,8 +445,8 @@ __device__ __forceinline__ void mp_harmonics_reg(const DevComp& c, int k, double
             else MPPtr<R>::template load<GEN>(rec, ac);
             rec += has_sin ? 2 * MPPtr<R>::REC : MPPtr<R>::REC;
             const R ll1 = R(L * (L + 1));
-            mp_col_acc<MODE, R>(gc, ac, sp, dw, ew, Pc, dPc, ll1);
-            if (has_sin) mp_col_acc<MODE, R>(gs, as, sp, dw, ew, Pc, dPc, ll1);
+            mp_col_acc<MODE, R>(gc, ac, sp, Pc, dPc, ll1);
+            if (has_sin) mp_col_acc<MODE, R>(gs, as, sp, Pc, dPc, ll1);
         };
         // even l only: Q_l = (cos^2 + A_l) Q_{l-2} + B_l Q_{l-4} (one step per stored l)
         const int ts = m * AGB_SKIP_N;
@@ -517,10 +521,8 @@ __device__ __forceinline__ void mp_harmonics_reg2(const DevComp& c1, const DevCo
     constexpr bool NEED_ANG2 = MODE == AGB_MODE_HESS;
     const bool near_pole = sth_d < 1.0e-10;
     const R s = (R)s_d;
-    R sp[6], dw[6], ew[6];
+    R sp[6];
     sp[0] = R(1); sp[1] = s; sp[2] = s * s; sp[3] = sp[2] * s; sp[4] = sp[2] * sp[2]; sp[5] = sp[4] * s;
-    dw[0] = R(0); dw[1] = R(1); dw[2] = R(2) * s; dw[3] = R(3) * sp[2]; dw[4] = R(4) * sp[3]; dw[5] = R(5) * sp[4];
-    ew[0] = R(0); ew[1] = R(0); ew[2] = R(2); ew[3] = R(6) * s; ew[4] = R(12) * sp[2]; ew[5] = R(20) * sp[3];
     const R cth = (R)cth_d, sth = (R)sth_d;
     const R cc2 = (R)(cth_d * cth_d), w2 = (R)(-2.0 * cth_d * sth_d);
     const R inv_sth = near_pole ? R(0) : (R)(1.0 / sth_d);
@@ -574,11 +576,11 @@ __device__ __forceinline__ void mp_harmonics_reg2(const DevComp& c1, const DevCo
             rec1 += has_sin ? 2 * MPPtr<R>::REC : MPPtr<R>::REC;
             rec2 += has_sin ? 2 * MPPtr<R>::REC : MPPtr<R>::REC;
             const R ll1 = R(L * (L + 1));
-            mp_col_acc<MODE, R>(gc1, ac1, sp, dw, ew, Pc, dPc, ll1);
-            mp_col_acc<MODE, R>(gc2, ac2, sp, dw, ew, Pc, dPc, ll1);
+            mp_col_acc<MODE, R>(gc1, ac1, sp, Pc, dPc, ll1);
+            mp_col_acc<MODE, R>(gc2, ac2, sp, Pc, dPc, ll1);
             if (has_sin) {
-                mp_col_acc<MODE, R>(gs1, as1, sp, dw, ew, Pc, dPc, ll1);
-                mp_col_acc<MODE, R>(gs2, as2, sp, dw, ew, Pc, dPc, ll1);
+                mp_col_acc<MODE, R>(gs1, as1, sp, Pc, dPc, ll1);
+                mp_col_acc<MODE, R>(gs2, as2, sp, Pc, dPc, ll1);
             }
         };
         const int ts = m * AGB_SKIP_N;
