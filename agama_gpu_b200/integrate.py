@@ -236,19 +236,28 @@ class Leapfrog:
         n, j = divmod(int(g), self.S)
         return self.t0 + n * self.dt + (self._sub[j - 1][2] if j else 0.0)
 
-    def _substep(self, x, v, F, g: int) -> None:
-        n, j = divmod(int(g), self.S)
-        dtj, hj, off = self._sub[j]
-        self._kd(x, v, F, 0.0, hj, dtj, 6)
-        self._force_at(x, n, off, F)
-        inc = 8 if (j == self.S - 1 and self._timed(x)) else 0
-        self._kd(x, v, F, hj, 0.0, 0.0, 1 | inc)
+    def _substeps(self, x, v, F, g0: int, n: int, before=None) -> None:
+        """n substeps from substep g0 on; F holds the force at x on entry and at the end.
+        The half-kick that ends a substep and the kick and drift that begin the next one
+        are one launch (the same updates in the same order).  before(g) is called with
+        x, v and F at the start of substep g, except that v still lacks the half-kick of
+        substep g - 1 (g > g0)."""
+        h_end, inc = 0.0, 0
+        for g in range(int(g0), int(g0) + int(n)):
+            step, j = divmod(g, self.S)
+            dtj, hj, off = self._sub[j]
+            if before is not None:
+                before(g)
+            self._kd(x, v, F, h_end, hj, dtj, (6 if g == g0 else 7) | inc)
+            self._force_at(x, step, off, F)
+            h_end, inc = hj, 8 if (j == self.S - 1 and self._timed(x)) else 0
+        if n > 0:
+            self._kd(x, v, F, h_end, 0.0, 0.0, 1 | inc)
 
-    def _step(self, x, v, F, n: int) -> None:
-        """One step from step index n, time t0 + n dt (all S substeps); with device
-        leaves the step counter must hold n and ends at n + 1."""
-        for g in range(int(n) * self.S, (int(n) + 1) * self.S):
-            self._substep(x, v, F, g)
+    def _steps(self, x, v, F, n0: int, n: int) -> None:
+        """n steps from step index n0, time t0 + n0 dt (S substeps each); with device
+        leaves the step counter must hold n0 and ends at n0 + n."""
+        self._substeps(x, v, F, int(n0) * self.S, int(n) * self.S)
 
     def _advance(self, x, v, F, n0: int, n_steps: int) -> None:
         """n_steps steps from step index n0 (time t0 + n0 dt)."""
@@ -256,8 +265,7 @@ class Leapfrog:
             return
         self._set_step(x, n0)
         if not self._graphs(x):
-            for k in range(n_steps):
-                self._step(x, v, F, n0 + k)
+            self._steps(x, v, F, n0, n_steps)
             return
         key = (x.data_ptr(), v.data_ptr(), F.data_ptr(), x.shape[0],
                getattr(self.pot, "plan_generation", 0), _consts_epoch(self.pot))
@@ -267,8 +275,7 @@ class Leapfrog:
         full, rest = divmod(n_steps, self.graph_steps)
         for _ in range(full):
             self._graph.replay()        # advances the device step counter itself
-        for k in range(rest):
-            self._step(x, v, F, n0 + full * self.graph_steps + k)
+        self._steps(x, v, F, n0 + full * self.graph_steps, rest)
 
     def _capture(self, x, v, F, n0: int) -> None:
         # warm-up on a side stream (allocator pools, lazy module loading), then capture;
@@ -277,15 +284,13 @@ class Leapfrog:
         s = torch.cuda.Stream(device=x.device)
         s.wait_stream(torch.cuda.current_stream(x.device))
         with torch.cuda.stream(s):
-            for k in range(2):
-                self._step(x, v, F, n0 + k)
+            self._steps(x, v, F, n0, 2)
         torch.cuda.current_stream(x.device).wait_stream(s)
         x.copy_(xs); v.copy_(vs); F.copy_(Fs)
         self._set_step(x, n0)
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):
-            for k in range(self.graph_steps):
-                self._step(x, v, F, n0 + k)
+            self._steps(x, v, F, n0, self.graph_steps)
         x.copy_(xs); v.copy_(vs); F.copy_(Fs)
         self._set_step(x, n0)
         self._graph = g
@@ -348,9 +353,7 @@ class Leapfrog:
             # every substep's positions in one allocation [substep][particle][3]; the
             # adjoint re-computes nothing and needs no velocities
             store = torch.empty((G + 1,) + tuple(x.shape), dtype=torch.float64, device=x.device)
-            for g in range(G):
-                store[g].copy_(x)
-                self._substep(x, v, F, g)
+            self._substeps(x, v, F, 0, G, before=lambda g: store[g].copy_(x))
             store[G].copy_(x)
             ckpts = [(g, store[g], None) for g in range(G)]
             ckpts.append((G, store[G], v.clone()))
@@ -536,9 +539,12 @@ class Leapfrog:
                 n_s, j_s = divmod(s, S)
                 self._set_step(x, n_s)
                 self._force_at(x, n_s, self._sub[j_s - 1][2] if j_s else 0.0, F)
+                def keep(g, s=s, X=X, x=x):
+                    if g > s:
+                        X[g - s - 1].copy_(x)
+                self._substeps(x, v, F, s, last - s, before=keep)
+                X[last - s - 1].copy_(x)
                 for g in range(s, last):
-                    self._substep(x, v, F, g)
-                    X[g - s].copy_(x)
                     pos[g + 1] = X[g - s]
             for g in range(e - 1, s - 1, -1):
                 if fused(pos[g + 1], g):

@@ -219,7 +219,7 @@ def particle_spray(pot, x_p, v_p, mass: float, t_end: float, n_steps: int, dt: f
     rec[n_steps, 0].copy_(xb[0])
     rec[n_steps, 1].copy_(vb[0])
     for n in range(n_steps):
-        back._step(xb, vb, Fb, n)
+        back._steps(xb, vb, Fb, n, 1)
         rec[n_steps - 1 - n, 0].copy_(xb[0])
         rec[n_steps - 1 - n, 1].copy_(vb[0])
     times = t_start + dt * np.arange(n_steps + 1, dtype=np.float64)
@@ -287,7 +287,7 @@ def integrate_releases(pot, x_release: torch.Tensor, v_release: torch.Tensor, re
             g = n * S + j
             if st is not None:
                 st[offsets[g]:offsets[g] + a].copy_(x[:a])
-            integ._substep(x[:a], v[:a], F[:a], g)
+            integ._substeps(x[:a], v[:a], F[:a], g, 1)
     t_release = torch.as_tensor(np.repeat(float(t_start) + dt * rel_steps, 2), device=dev)
     return Stream(x=x, v=v, t_release=t_release, x_release=x_rel, v_release=v_rel, track=None,
                   r_jacobi=None, _integ=integ, _counts=counts, _store=st,
