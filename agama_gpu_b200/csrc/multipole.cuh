@@ -333,6 +333,65 @@ __device__ __forceinline__ void mp_col_acc(MPCol<R>& g, const R a[6], const R sp
     if (NEED_ANG) g.VT = fma(C, dY, g.VT);
 }
 
+// Two FP32 lanes in one instruction, each rounded as the scalar instruction rounds it.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
+{
+    float2 d;
+    asm("{ .reg .b64 x, y, z, w;\n\t"
+        "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+        "fma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w; }"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+
+// Both trig columns of one harmonic m > 0.  FP32: the cos and sin columns, whose coefficients
+// are stored interleaved, are the two lanes of packed multiply-adds.  The FP32 walk is bound by
+// issue (59-73 % of the slots, the FMA pipe at 32-39 %), and these halve 24 of its 29
+// multiply-adds per harmonic: 48 halos in one batch 1348 -> 1270 us, the 4M-point
+// time-dependent tree 4150 -> 3940 (with the two-table walk below unrolled by 4 rather than 2,
+// which alone loses: 4050 -> 4170).  The adjoint walk keeps one column at a time: packed it
+// took 2.74 ms against 2.60 (131072 orbits, 8 steps, lmax 16).
+template <int MODE, typename R>
+__device__ __forceinline__ void mp_col_acc_cs(MPCol<R>& gc, MPCol<R>& gs, const R ac[6],
+                                              const R as[6], const R sp[6], R Y, R dY, R ll1)
+{
+    if constexpr (std::is_same<R, float>::value) {
+        constexpr bool NEED_B = MODE != AGB_MODE_POT;
+        constexpr bool NEED_D = MODE == AGB_MODE_HESS || MODE == AGB_MODE_DENS;
+        constexpr bool NEED_ANG = MODE == AGB_MODE_GRAD || MODE == AGB_MODE_HESS;
+        const float2 x = {sp[1], sp[1]}, y = {Y, Y}, dy = {dY, dY};
+        float2 a[6];
+        #pragma unroll
+        for (int j = 0; j < 6; ++j) a[j] = {ac[j], as[j]};
+        float2 p = fma2(a[5], x, a[4]), d = a[5], e = a[5];
+        #pragma unroll
+        for (int j = 3; j >= 0; --j) {
+            if (NEED_B) d = fma2(d, x, p);
+            p = fma2(p, x, a[j]);
+            if (NEED_D && j > 0) e = fma2(e, x, d);
+        }
+        auto acc = [](float& c, float& s, float2 u, float2 v) {
+            const float2 r = fma2(u, v, {c, s});
+            c = r.x;
+            s = r.y;
+        };
+        acc(gc.V, gs.V, p, y);
+        if (NEED_B) {
+            acc(gc.VR, gs.VR, d, y);
+            if (MODE == AGB_MODE_HESS) acc(gc.VRT, gs.VRT, d, dy);
+        }
+        if (NEED_D) {
+            acc(gc.VRR, gs.VRR, e, y);
+            acc(gc.L, gs.L, {ll1 * p.x, ll1 * p.y}, y);
+        }
+        if (NEED_ANG) acc(gc.VT, gs.VT, p, dy);
+    } else {
+        mp_col_acc<MODE, R>(gc, ac, sp, Y, dY, ll1);
+        mp_col_acc<MODE, R>(gs, as, sp, Y, dY, ll1);
+    }
+}
+
 // the group's Y/sin and d2Y/dtheta2 sums from its accumulators (see above)
 template <int MODE, typename R>
 __device__ __forceinline__ void mp_col_finish(MPCol<R>& g, R inv_sth, R q1, R np1, R cot, R m2)
@@ -445,8 +504,8 @@ __device__ __forceinline__ void mp_harmonics_reg(const DevComp& c, int k, double
             else MPPtr<R>::template load<GEN>(rec, ac);
             rec += has_sin ? 2 * MPPtr<R>::REC : MPPtr<R>::REC;
             const R ll1 = R(L * (L + 1));
-            mp_col_acc<MODE, R>(gc, ac, sp, Pc, dPc, ll1);
-            if (has_sin) mp_col_acc<MODE, R>(gs, as, sp, Pc, dPc, ll1);
+            if (has_sin) mp_col_acc_cs<MODE, R>(gc, gs, ac, as, sp, Pc, dPc, ll1);
+            else mp_col_acc<MODE, R>(gc, ac, sp, Pc, dPc, ll1);
         };
         // even l only: Q_l = (cos^2 + A_l) Q_{l-2} + B_l Q_{l-4} (one step per stored l)
         const int ts = m * AGB_SKIP_N;
@@ -576,11 +635,12 @@ __device__ __forceinline__ void mp_harmonics_reg2(const DevComp& c1, const DevCo
             rec1 += has_sin ? 2 * MPPtr<R>::REC : MPPtr<R>::REC;
             rec2 += has_sin ? 2 * MPPtr<R>::REC : MPPtr<R>::REC;
             const R ll1 = R(L * (L + 1));
-            mp_col_acc<MODE, R>(gc1, ac1, sp, Pc, dPc, ll1);
-            mp_col_acc<MODE, R>(gc2, ac2, sp, Pc, dPc, ll1);
             if (has_sin) {
-                mp_col_acc<MODE, R>(gs1, as1, sp, Pc, dPc, ll1);
-                mp_col_acc<MODE, R>(gs2, as2, sp, Pc, dPc, ll1);
+                mp_col_acc_cs<MODE, R>(gc1, gs1, ac1, as1, sp, Pc, dPc, ll1);
+                mp_col_acc_cs<MODE, R>(gc2, gs2, ac2, as2, sp, Pc, dPc, ll1);
+            } else {
+                mp_col_acc<MODE, R>(gc1, ac1, sp, Pc, dPc, ll1);
+                mp_col_acc<MODE, R>(gc2, ac2, sp, Pc, dPc, ll1);
             }
         };
         const int ts = m * AGB_SKIP_N;
@@ -604,13 +664,13 @@ __device__ __forceinline__ void mp_harmonics_reg2(const DevComp& c1, const DevCo
             if (PAR == 2) {
                 Pp = (m == 0) ? seed : R(0);
                 dPp = R(0);
-                #pragma unroll 2
+                #pragma unroll 4
                 for (l = l0 + 2; l <= lmax; l += 2) {
                     skip2(l);
                     acc(l, has_sin);
                 }
             } else {
-                #pragma unroll 2
+                #pragma unroll 4
                 for (l = l0 + 1; l <= lmax; ++l) {
                     step(l);
                     acc(l, has_sin);
