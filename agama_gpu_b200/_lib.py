@@ -7,6 +7,7 @@ CUDA device raises RuntimeError from the first evaluation.
 from __future__ import annotations
 
 import ctypes
+import struct
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "libagb.so"
@@ -77,6 +78,11 @@ class AgbLeaf(ctypes.Structure):
         ("gamma", ctypes.c_double * 3),
         ("ampl", ctypes.c_double),
     ]
+
+
+# one AgbLeaf record: pack_leaf(comp, sigma, gamma x, y, z, ampl)
+pack_leaf = struct.Struct("@i4x5d").pack
+assert struct.calcsize("@i4x5d") == ctypes.sizeof(AgbLeaf)
 
 
 MAX_LEAF_OPS = 6
