@@ -19,14 +19,21 @@
 // depend on it.
 //
 // Calls of at most AGB_BIN_SMALL points are sorted by bin_small in ONE launch: the
-// passes' launches and the gaps between them cost more than the work there.
+// passes' launches and the gaps between them cost more than the work there.  Evaluations of
+// at most AGB_BIN_SLICED points take it too, in slices that are sorted by themselves, and
+// write their outputs in place: the warps' runs of one interval stay long enough, and neither
+// the passes nor the output gather are launched.  FP64 calls in three passes / in slices, us:
+// densities at lmax 20 68 / 64 (40k points), 128 / 124 (100k); potentials at lmax 16 39 / 36,
+// 66 / 63; mixed forces at lmax 16 41 / 37, 69 / 65.  Beyond, the intervals' rows are read
+// anew in every slice: 103 / 103 at 300k, 172 / 179 at 524k, 289 / 313 at 1M.
 #pragma once
 #include <cooperative_groups.h>
 #include "agb_dev.cuh"
 
 #define AGB_BIN_TILE_MAX 4096      // points per block in passes 1 and 3 (at most)
 #define AGB_MAX_BINS 8192
-#define AGB_BIN_SMALL 32768        // most points of bin_small: 8 blocks x 1024 threads x 4
+#define AGB_BIN_SMALL 32768        // most points of a slice of bin_small: 8 blocks x 1024 threads x 4
+#define AGB_BIN_SLICED 131072      // most points of an evaluation that is sorted in slices
 #define AGB_BIN_SMALL_BINS 1024    // and most bins: one thread each in the scan
 
 struct BinKey {
@@ -135,14 +142,14 @@ bin_scatter(const double* __restrict__ xyz, long long n, int tile, int n_bins,
     }
 }
 
-// The whole sort in one launch: a cluster of 8 blocks, each with an eighth of the points, at
-// most 4 a thread, kept in registers between counting and placing.  The blocks read each
+// The whole sort in one launch: a cluster of 8 blocks per slice of the points, each block with an
+// eighth of it, at most 4 points a thread, kept in registers between counting and placing.  The blocks read each
 // other's histograms through distributed shared memory; every block scans the bins itself.
 // Bound by the latency of its steps (the log of a point's radius, two cluster barriers, the
 // scan), not by bandwidth.
 #define AGB_BIN_SMALL_BLOCKS 8
 __global__ void __cluster_dims__(AGB_BIN_SMALL_BLOCKS, 1, 1) __launch_bounds__(1024)
-bin_small(const double* __restrict__ xyz, int n, BinKey b, int n_bins, int* __restrict__ keys,
+bin_small(const double* __restrict__ xyz, int n, int slice, BinKey b, int n_bins, int* __restrict__ keys,
           int* __restrict__ perm, double* __restrict__ xyz_sorted)
 {
     namespace cg = cooperative_groups;
@@ -155,6 +162,10 @@ bin_small(const double* __restrict__ xyz, int n, BinKey b, int n_bins, int* __re
     }
     hist[t] = 0;
     __syncthreads();
+    // this cluster's slice of the points, sorted in its own rows
+    const int first = (int)(blockIdx.x / AGB_BIN_SMALL_BLOCKS) * slice;
+    n = min(slice, n - first);
+    const double* src = xyz + 3LL * first;
     const int per = (n + AGB_BIN_SMALL_BLOCKS - 1) / AGB_BIN_SMALL_BLOCKS;
     const int lo = rank * per, hi = min(lo + per, n);
     double p[4][3];
@@ -163,7 +174,7 @@ bin_small(const double* __restrict__ xyz, int n, BinKey b, int n_bins, int* __re
     for (int j = 0; j < 4; ++j) {
         const int i = lo + t + 1024 * j;
         if (i >= hi) continue;
-        p[j][0] = xyz[3 * i]; p[j][1] = xyz[3 * i + 1]; p[j][2] = xyz[3 * i + 2];
+        p[j][0] = src[3 * i]; p[j][1] = src[3 * i + 1]; p[j][2] = src[3 * i + 2];
         key[j] = bin_of(b, p[j][0], p[j][1], p[j][2]);
         at[j] = atomicAdd(&hist[key[j]], 1);
     }
@@ -202,11 +213,10 @@ bin_small(const double* __restrict__ xyz, int n, BinKey b, int n_bins, int* __re
     for (int j = 0; j < 4; ++j) {
         const int i = lo + t + 1024 * j;
         if (i >= hi) continue;
-        const int pos = base[key[j]] + at[j];
-        if (perm) perm[pos] = i;
-        keys[i] = pos;
-        xyz_sorted[3 * pos] = p[j][0];
-        xyz_sorted[3 * pos + 1] = p[j][1];
-        xyz_sorted[3 * pos + 2] = p[j][2];
+        const int pos = first + base[key[j]] + at[j];
+        if (perm) perm[pos] = first + i;
+        keys[first + i] = pos;
+        double* o = xyz_sorted + 3LL * pos;
+        o[0] = p[j][0]; o[1] = p[j][1]; o[2] = p[j][2];
     }
 }

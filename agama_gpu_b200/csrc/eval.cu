@@ -411,6 +411,7 @@ struct BinPlan {
     BinKey key;
     int n_bins;
     int leaf;          // the keyed leaf
+    bool one;          // sorted by bin_small, in slices of AGB_BIN_SMALL points
 };
 
 // What a point gains (ns) when the walk of this Multipole reads its records as broadcasts
@@ -435,9 +436,8 @@ static double sort_gain(const agb_component& c, int mode)
 // E.g. FP64 forces, sorted / unsorted: lmax 8 44 / 32 us at 100k points; lmax 12 103 / 108 at
 // 300k; lmax 16 45 / 46 us at 40k, 75 / 90 at 100k, 1490 / 2365 at 4M.  mode < 0: any mode
 // (workspace sizes).
-static bool sort_pays(double gain, int64_t n, int n_bins, int mode)
+static bool sort_pays(double gain, int64_t n, bool small, int mode)
 {
-    const bool small = n <= AGB_BIN_SMALL && n_bins <= AGB_BIN_SMALL_BINS;
     const double cost = mode == AGB_MODE_HESS ? 0.16 : 0.06;
     return (double)n * (gain - cost) > (small ? 5000.0 : 6000.0);
 }
@@ -460,6 +460,8 @@ static BinPlan plan_binning(const agb_component* comps, const agb_leaf* leaves, 
     }
     if (best < 0 || best_lm < 2) return b;
     const agb_component& c = comps[leaves[best].comp];
+    // sums over an interval's points (adjoints, table gradients) want long runs: one slice
+    b.one = n <= (eval ? AGB_BIN_SLICED : AGB_BIN_SMALL) && c.n_int + 2 <= AGB_BIN_SMALL_BINS;
     if (eval && !(out_flags & AGB_OUT_BIN_ALWAYS)) {
         double gain = 0.0;            // of every Multipole in the keyed one's frame
         for (int L = 0; L < n_leaves; ++L) {
@@ -468,7 +470,7 @@ static BinPlan plan_binning(const agb_component* comps, const agb_leaf* leaves, 
                 !memcmp(leaves[L].gamma, leaves[best].gamma, sizeof(leaves[L].gamma)))
                 gain += sort_gain(q, mode < 0 ? AGB_MODE_POT : mode);
         }
-        if (!sort_pays(gain, n, c.n_int + 2, mode)) return b;
+        if (!sort_pays(gain, n, b.one && n <= AGB_BIN_SMALL, mode)) return b;
     }
     b.on = true;
     b.leaf = best;
@@ -597,9 +599,11 @@ static int run_binning(EvalArgs& a, const BinPlan& b, const double* xyz, int64_t
         cudaFuncSetAttribute(bin_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * AGB_MAX_BINS);
         g_bin_attr_set.fetch_or(bit, std::memory_order_release);
     }
-    if (n <= AGB_BIN_SMALL && b.n_bins <= AGB_BIN_SMALL_BINS) {
-        bin_small<<<AGB_BIN_SMALL_BLOCKS, 1024, 0, st>>>(xyz, (int)n, b.key, b.n_bins, keys,
-                                                         with_perm ? perm : nullptr, xs);
+    if (b.one) {
+        const int slices = (int)((n + AGB_BIN_SMALL - 1) / AGB_BIN_SMALL);
+        const int slice = (int)(((n + slices - 1) / slices + 31) / 32 * 32);
+        bin_small<<<slices * AGB_BIN_SMALL_BLOCKS, 1024, 0, st>>>(
+            xyz, (int)n, slice, b.key, b.key.n_int + 2, keys, with_perm ? perm : nullptr, xs);
         a.xyz = xs;
         a.perm = with_perm ? perm : nullptr;
         return check_launch("bin_small");
@@ -651,7 +655,7 @@ static int eval_impl(const agb_component* comps, int n_comps, const agb_leaf* le
     // sorted-order output staging when the workspace has room for it (always for
     // agb_eval's own allocation and for workspaces sized by agb_eval_workspace_bytes)
     const size_t staged = ws_bytes_staged(b, n);
-    const bool stage = b.on && n > AGB_BIN_SMALL && (own_ws || (workspace && workspace_bytes >= staged));
+    const bool stage = b.on && !b.one && (own_ws || (workspace && workspace_bytes >= staged));
     const size_t need = stage ? staged : ws_bytes(b, n);
     void* ws = workspace;
     if (need) {
@@ -1074,7 +1078,7 @@ extern "C" int agb_eval_timed(const agb_component* comps, int n_comps, const agb
             return set_err(AGB_ERR_ARG, "agb_eval_timed: workspace of %zu bytes is smaller than "
                            "the %zu bytes agb_eval_timed_workspace_bytes asks for",
                            workspace_bytes, need + TP_LEAF_BYTES);
-        const bool stage = n > AGB_BIN_SMALL && room >= staged;
+        const bool stage = !b.one && room >= staged;
         const bool vjp = mode == AGB_MODE_VJP || mode == AGB_MODE_VJPF;
         if ((rc = run_binning(a, b, xyz, n, ws, st, !stage || vjp))) return rc;
         if (stage) {

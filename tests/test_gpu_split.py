@@ -76,3 +76,13 @@ def test_one_launch_sort(n):
     one = _all(pot, x, "fp64", _lib.OUT_NO_BINNING | 1 << _lib.OUT_GRID_SHIFT)
     _close(_all(pot, x, "fp64", _lib.OUT_BIN_ALWAYS), one)
     _close(_all(pot, x, "fp64", _lib.OUT_BIN_ALWAYS | 1 << _lib.OUT_GRID_SHIFT), one)
+
+
+@pytest.mark.parametrize("n", [32768, 32769, 65569, 131072, 131073])
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_sorted_in_slices_equals_unsorted(n, prec):
+    """Edges of the slices and of their rule; the order of the points changes no bit."""
+    from agama_gpu_b200 import _lib
+    pot, x = _halo(6, True), _points(n)
+    for a, b in zip(_all(pot, x, prec, _lib.OUT_NO_BINNING), _all(pot, x, prec, 4)):
+        assert (a == b).all()
