@@ -434,12 +434,16 @@ static double sort_gain(const agb_component& c, int mode)
 // in one launch (bin_small), and 0.06 ns a point (0.16 with Hessians); half of the 13 us are
 // gained back by the kernel's coalesced stores and warmer rows, so the line lies at 6 us.
 // E.g. FP64 forces, sorted / unsorted: lmax 8 44 / 32 us at 100k points; lmax 12 103 / 108 at
-// 300k; lmax 16 45 / 46 us at 40k, 75 / 90 at 100k, 1490 / 2365 at 4M.  mode < 0: any mode
-// (workspace sizes).
+// 300k; lmax 16 45 / 46 us at 40k, 75 / 90 at 100k, 1490 / 2365 at 4M.
 static bool sort_pays(double gain, int64_t n, bool small, int mode)
 {
     const double cost = mode == AGB_MODE_HESS ? 0.16 : 0.06;
     return (double)n * (gain - cost) > (small ? 5000.0 : 6000.0);
+}
+
+static bool sortable(const agb_component& c)
+{
+    return c.kind == AGB_KIND_MULTIPOLE && c.n_lm >= 2 && c.n_int + 2 <= AGB_MAX_BINS;
 }
 
 // eval: an evaluation in `mode` (else an adjoint or table gradient, whose sums need the order)
@@ -453,12 +457,12 @@ static BinPlan plan_binning(const agb_component* comps, const agb_leaf* leaves, 
     int best = -1, best_lm = 0;
     for (int L = 0; L < n_leaves; ++L) {
         const agb_component& c = comps[leaves[L].comp];
-        if (c.kind == AGB_KIND_MULTIPOLE && c.n_lm > best_lm && c.n_int + 2 <= AGB_MAX_BINS) {
+        if (sortable(c) && c.n_lm > best_lm) {
             best = L;
             best_lm = c.n_lm;
         }
     }
-    if (best < 0 || best_lm < 2) return b;
+    if (best < 0) return b;
     const agb_component& c = comps[leaves[best].comp];
     // sums over an interval's points (adjoints, table gradients) want long runs: one slice
     b.one = n <= (eval ? AGB_BIN_SLICED : AGB_BIN_SMALL) && c.n_int + 2 <= AGB_BIN_SMALL_BINS;
@@ -468,7 +472,7 @@ static BinPlan plan_binning(const agb_component* comps, const agb_leaf* leaves, 
             const agb_component& q = comps[leaves[L].comp];
             if (q.kind == AGB_KIND_MULTIPOLE && leaves[L].sigma == leaves[best].sigma &&
                 !memcmp(leaves[L].gamma, leaves[best].gamma, sizeof(leaves[L].gamma)))
-                gain += sort_gain(q, mode < 0 ? AGB_MODE_POT : mode);
+                gain += sort_gain(q, mode);
         }
         if (!sort_pays(gain, n, b.one && n <= AGB_BIN_SMALL, mode)) return b;
     }
@@ -500,6 +504,27 @@ static size_t ws_bytes_staged(const BinPlan& b, int64_t n)
 {
     if (!b.on) return 0;
     return ws_bytes(b, n) + al256(8 * (size_t)AGB_STAGE_MAX_REC * (size_t)n);
+}
+
+// Scratch that serves every evaluation of at most n points over this component array: the
+// rule that decides on sorting looks at the leaves, which change with time, and at n (a call of
+// fewer points may sort where one of more does not), so the bound looks at neither the leaves
+// nor the rule.
+static size_t ws_bound(const agb_component* comps, int n_comps, int64_t n, int out_flags)
+{
+    if ((out_flags & AGB_OUT_NO_BINNING) || n < 1 || n > 0x7fffffffLL) return 0;
+    for (int c = 0; c < n_comps; ++c)
+        if (sortable(comps[c]))
+            return 2 * al256(4 * (size_t)n) + al256(24 * (size_t)n) + 2 * al256(4 * (size_t)AGB_MAX_BINS)
+                   + al256(8 * (size_t)AGB_STAGE_MAX_REC * (size_t)n);
+    return 0;
+}
+
+// Calls below AGB_BIN_MIN_POINTS need no scratch: given less than the sort takes, they are
+// evaluated in input order (each point's result is the same).
+static bool sort_optional(int64_t n, int out_flags)
+{
+    return n < AGB_BIN_MIN_POINTS && !(out_flags & AGB_OUT_BIN_ALWAYS);
 }
 
 static int validate(const agb_component* comps, int n_comps, const agb_leaf* leaves, int n_leaves,
@@ -651,7 +676,10 @@ static int eval_impl(const agb_component* comps, int n_comps, const agb_leaf* le
     a.gphi = g_vjp_phi; a.gforce = g_vjp_force;
     if ((rc = pack_args(a, comps, n_comps, leaves, n_leaves, precision))) return rc;
 
-    const BinPlan b = plan_binning(comps, leaves, n_leaves, n, out_flags, 1, mode);
+    BinPlan b = plan_binning(comps, leaves, n_leaves, n, out_flags, 1, mode);
+    if (sort_optional(n, out_flags) &&
+        (own_ws || !workspace || ((uintptr_t)workspace & 255u) || workspace_bytes < ws_bytes(b, n)))
+        b.on = false;
     // sorted-order output staging when the workspace has room for it (always for
     // agb_eval's own allocation and for workspaces sized by agb_eval_workspace_bytes)
     const size_t staged = ws_bytes_staged(b, n);
@@ -693,7 +721,18 @@ extern "C" size_t agb_eval_workspace_bytes(const agb_component* comps, int n_com
     if (!comps || !leaves || n_leaves < 1 || n_comps < 1) return 0;
     for (int L = 0; L < n_leaves; ++L)
         if (leaves[L].comp < 0 || leaves[L].comp >= n_comps) return 0;
-    return ws_bytes_staged(plan_binning(comps, leaves, n_leaves, n, out_flags, 1), n);
+    return ws_bound(comps, n_comps, n, out_flags);
+}
+
+extern "C" size_t agb_eval_scratch_bytes(const agb_component* comps, int n_comps,
+                                         const agb_leaf* leaves, int n_leaves, int64_t n, int mode,
+                                         int out_flags)
+{
+    if (!comps || !leaves || n_leaves < 1 || n_comps < 1) return 0;
+    for (int L = 0; L < n_leaves; ++L)
+        if (leaves[L].comp < 0 || leaves[L].comp >= n_comps) return 0;
+    const BinPlan b = plan_binning(comps, leaves, n_leaves, n, out_flags, 1, mode);
+    return b.one ? ws_bytes(b, n) : ws_bytes_staged(b, n);
 }
 
 extern "C" int64_t agb_eval_wave_points(const agb_component* comps, int n_comps,
@@ -1019,9 +1058,7 @@ extern "C" size_t agb_eval_timed_workspace_bytes(const agb_component* comps, int
     if (!comps || !p || n_comps < 1) return 0;
     for (int i = 0; i < p->n; ++i)
         if (p->max_comp[i] >= n_comps) return 0;
-    agb_leaf lv[AGB_MAX_LEAVES];
-    tp_template_leaves(p, lv);
-    return TP_LEAF_BYTES + ws_bytes_staged(plan_binning(comps, lv, p->n, n, out_flags, 1), n);
+    return TP_LEAF_BYTES + ws_bound(comps, n_comps, n, out_flags);
 }
 
 extern "C" int agb_eval_timed(const agb_component* comps, int n_comps, const agb_time_plan* p,
@@ -1070,6 +1107,7 @@ extern "C" int agb_eval_timed(const agb_component* comps, int n_comps, const agb
     char* ws = (char*)workspace + TP_LEAF_BYTES;
     const size_t room = workspace_bytes - TP_LEAF_BYTES;
     BinPlan b = plan_binning(comps, lv, p->n, n, out_flags, 1, mode);
+    if (sort_optional(n, out_flags) && room < ws_bytes(b, n)) b.on = false;
     if (b.on) {
         b.key.leaf = dl + b.leaf;
         const size_t staged = ws_bytes_staged(b, n);

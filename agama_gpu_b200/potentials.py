@@ -433,9 +433,8 @@ class _GPUPotBase:
             f |= tuned.get((mode, prec, int(n).bit_length()), 0)
         return f
 
-    def _workspace(self, cargs, n: int, dev: torch.device, flags: int):
-        nws = int(_lib.lib.agb_eval_workspace_bytes(cargs[0], cargs[1], cargs[2], cargs[3], n,
-                                                    flags))
+    def _workspace(self, cargs, n: int, dev: torch.device, flags: int, mode: int):
+        nws = int(_lib.lib.agb_eval_scratch_bytes(*cargs, n, mode, flags))
         return (torch.empty(nws, dtype=torch.uint8, device=dev) if nws else None), nws
 
     def _launch(self, arr: torch.Tensor, t: float, mode: int, want_phi: bool,
@@ -464,7 +463,7 @@ class _GPUPotBase:
         ptr = lambda a: None if a is None else a.data_ptr()  # noqa: E731
         stream = torch._C._cuda_getCurrentRawStream(dev.index)     # 0.1 us, a Stream object 2.2
         flags = self._flags(mode, prec, n)
-        ws, nws = self._workspace(cargs, n, dev, flags)
+        ws, nws = self._workspace(cargs, n, dev, flags, mode)
         rc = _lib.lib.agb_eval_ws(*cargs, arr.data_ptr(), n, mode, prec, ptr(phi), ptr(grad),
                                   ptr(hess), ptr(rho), flags, ptr(ws), nws,
                                   stream)
@@ -487,7 +486,7 @@ class _GPUPotBase:
         gp = None if g_phi is None else g_phi.to(device=dev, dtype=torch.float64).contiguous()
         gf = None if g_force is None else g_force.to(device=dev, dtype=torch.float64).contiguous()
         ptr = lambda a: None if a is None else a.data_ptr()  # noqa: E731
-        ws, nws = self._workspace(cargs, n, dev, 0)       # agb_eval_vjp sorts by default
+        ws, nws = self._workspace(cargs, n, dev, 0, _lib.MODE_VJP)   # agb_eval_vjp sorts by default
         stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
         if force_out is None:
             rc = _lib.lib.agb_eval_vjp(*cargs, arr.data_ptr(), n, prec, ptr(gp), ptr(gf),
@@ -751,10 +750,10 @@ class _GPUPotBase:
             return self._eval_host_run(src, host, want, n, chunk, t, mode, pot, dev, pipe)
 
     def _eval_host_run(self, src, host, want, n, chunk, t, mode, pot, dev, pipe):
-        # The chunk layout, launch flags and workspace size depend only on the call's
-        # shape, so they are kept per shape on the object; the first chunk's copy-in is
-        # queued before the tree's arguments at t are formed (the host's remaining work
-        # before the first launch), so that copy overlaps it.  Each chunk then costs the
+        # The chunk layout and launch flags depend only on the call's shape, so they are
+        # kept per shape on the object; the first chunk's copy-in is queued before the
+        # tree's arguments at t are formed and the scratch they need is asked for (the
+        # host's remaining work before the first launch), so that copy overlaps it.  Each chunk then costs the
         # host one C call and the first kernel follows its copy directly.
         prec = _PRECISIONS[self.precision or _default_precision]
         tuned = self.__dict__.get("_tuned") or {}
@@ -774,15 +773,12 @@ class _GPUPotBase:
                 # a launch takes the same number of passes (unless a tuned shape is set)
                 flags = {m: f if (f >> _lib.OUT_GRID_SHIFT) & 15 or (f >> _lib.OUT_PPT_SHIFT) & 15
                          else f | (1 << _lib.OUT_GRID_SHIFT) for m, f in flags.items()}
-            nws = max((int(_lib.lib.agb_eval_workspace_bytes(cargs[0], cargs[1], cargs[2],
-                                                             cargs[3], m, flags[m]))
-                       for m in sizes), default=0)
             # the device buffers hold the largest chunk
-            plan = (bounds, max(sizes), flags, nws)
+            plan = (bounds, max(sizes), flags)
             if len(plans) >= 64:
                 plans.clear()
             plans[key] = plan
-        bounds, chunk, flags, nws = plan
+        bounds, chunk, flags = plan
         ptr = lambda a: None if a is None else a.data_ptr()  # noqa: E731
         cur = torch.cuda.current_stream(dev)
         s_in, s_cmp, s_out = pipe["streams"]
@@ -796,6 +792,8 @@ class _GPUPotBase:
             ev_in[0].record(s_in)
         if cargs is None:
             cargs = self._c_args(t, dev)
+        # the leaves at t decide which chunks sort
+        nws = max(int(_lib.lib.agb_eval_scratch_bytes(*cargs, m, mode, f)) for m, f in flags.items())
         ws = pipe["bufs"].get("ws")
         if nws and (ws is None or ws.numel() < nws):
             # allocated on the compute stream, the only one that uses it

@@ -94,7 +94,8 @@ extern "C" {
 /* the adjoint and table-gradient entries sort the points by the radial interval of
    the Multipole (a counting sort in device scratch) when there are at least this many;
    the evaluation entries sort where the estimated gain of the walk exceeds the cost of
-   the sort (more points for smaller tables; AGB_OUT_BIN_ALWAYS: always) */
+   the sort (more points for smaller tables; AGB_OUT_BIN_ALWAYS: always), below this many
+   points only in scratch that the caller gives */
 #define AGB_BIN_MIN_POINTS 16384
 
 /* component kinds */
@@ -221,13 +222,24 @@ int agb_eval(const agb_component* comps, int n_comps,
 
 /*
  * agb_eval with caller-provided device scratch for the interval sort (no
- * allocation inside).  workspace: 256-byte aligned, at least
- * agb_eval_workspace_bytes(...) bytes (0 when the call does not sort; then
- * workspace may be NULL).  The scratch is about 32 bytes per point.
+ * allocation inside).  workspace: 256-byte aligned, of
+ *  - agb_eval_workspace_bytes(...): enough for every call of at most n points with
+ *    this component array and these flags, whatever the leaves (a time-dependent
+ *    tree's change from call to call), the mode and the precision; 112 bytes per
+ *    point (32 for the sort, 80 for the outputs in sorted order) where a component
+ *    is a Multipole, else 0;
+ *  - or agb_eval_scratch_bytes(...): what this very call uses, 0 when it does not
+ *    sort (then workspace may be NULL).
+ * A call that sorts refuses less than the sort's 32 bytes per point, except below
+ * AGB_BIN_MIN_POINTS (without AGB_OUT_BIN_ALWAYS), where it then evaluates the
+ * points in input order.
  */
 size_t agb_eval_workspace_bytes(const agb_component* comps, int n_comps,
                                 const agb_leaf* leaves, int n_leaves, int64_t n,
                                 int out_flags);
+size_t agb_eval_scratch_bytes(const agb_component* comps, int n_comps,
+                              const agb_leaf* leaves, int n_leaves, int64_t n, int mode,
+                              int out_flags);
 int agb_eval_ws(const agb_component* comps, int n_comps,
                 const agb_leaf* leaves, int n_leaves,
                 const double* xyz, int64_t n, int mode, int precision,
@@ -558,8 +570,8 @@ int agb_time_plan_leaves(const agb_time_plan* plan, const int64_t* step, double 
 /*
  * agb_eval_ws with the plan's leaves at t = (t0 + (*step) * dt) + off computed on
  * the device in the same stream: no host value of t enters a launch.  The
- * workspace (agb_eval_timed_workspace_bytes) holds the device leaves and the
- * interval-sort scratch.
+ * workspace (agb_eval_timed_workspace_bytes: enough for every call of at most n
+ * points) holds the device leaves and the interval-sort scratch.
  */
 size_t agb_eval_timed_workspace_bytes(const agb_component* comps, int n_comps,
                                       const agb_time_plan* plan, int64_t n, int out_flags);

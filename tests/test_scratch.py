@@ -1,0 +1,93 @@
+"""Scratch of the evaluation entries: what is asked for serves every smaller call and every
+time, and calls that need none run without it."""
+import pytest
+
+
+def _descriptors(columns, nodes=50, n_leaves=1):
+    """Multipoles of so many columns in one frame, described as far as sizes look at them."""
+    from agama_gpu_b200 import _lib
+    comps = (_lib.AgbComponent * n_leaves)()
+    leaves = (_lib.AgbLeaf * n_leaves)()
+    for i in range(n_leaves):
+        comps[i].kind = _lib.KIND_MULTIPOLE
+        comps[i].n_lm, comps[i].n_int = columns, nodes - 1
+        leaves[i].comp, leaves[i].sigma, leaves[i].ampl = i, 1.0, 1.0
+    return comps, n_leaves, leaves, n_leaves
+
+
+SIZES = [1, 4999, 16383, 16384, 32768, 32769, 32868, 60000, 100003, 131072, 131073, 1 << 20,
+         (1 << 23) + 1]
+
+
+@pytest.mark.parametrize("lmax", [4, 6, 8, 10, 12, 16, 20, 32])
+def test_workspace_of_the_largest_call_serves_smaller_ones(lmax):
+    from agama_gpu_b200 import _lib
+    columns = (lmax // 2 + 1) * (lmax + 1)
+    one, two = _descriptors(columns), _descriptors(columns, n_leaves=2)
+    most = 0
+    for n in SIZES:
+        # two snapshots in use, or one of them
+        b = _lib.lib.agb_eval_workspace_bytes(*two, n, 0)
+        assert b == _lib.lib.agb_eval_workspace_bytes(two[0], 2, two[2], 1, n, 0) >= most
+        most = b
+        for args in (one, two):
+            for mode in range(5):
+                for flags in (0, _lib.OUT_BIN_ALWAYS):
+                    assert _lib.lib.agb_eval_scratch_bytes(*args, n, mode, flags) <= most
+    assert _lib.lib.agb_eval_workspace_bytes(*two, 10**6, _lib.OUT_NO_BINNING) == 0
+    assert _lib.lib.agb_eval_scratch_bytes(*two, 10**6, _lib.MODE_POT, _lib.OUT_NO_BINNING) == 0
+
+
+def _multipole(lmax, seed=3, nodes=50):
+    import agama_gpu_b200 as agb
+    from agama_gpu_b200.synthetic import nfw_multipole
+    return agb.MultipolePotentialGPU(nfw_multipole(lmax=lmax, n_nodes=nodes, seed=seed, amp=0.3))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [60000, 131072])
+@pytest.mark.parametrize("lmax", [6, 8, 12])
+def test_eval_host_at_a_snapshot_and_between(n, lmax):
+    import torch
+    import agama_gpu_b200 as agb
+    from agama_gpu_b200.synthetic import hernquist_points
+    pot = agb.EvolvingPotentialGPU([_multipole(lmax, s) for s in (1, 2, 3)], [0.0, 1.0, 2.0])
+    x = torch.from_numpy(hernquist_points(n, 10.0, 5))
+    xd = x.cuda()
+    for t in (0.0, 0.5, 1.0, 1.7, -1.0):
+        for want in (dict(pot=True), dict(pot=True, acc=True), dict(der=True)):
+            got, ref = pot.eval_host(x, t=t, **want), pot.eval(xd, t=t, **want)
+            for a, b in zip(*((v if isinstance(v, tuple) else (v,)) for v in (got, ref))):
+                # a chunk may take another kernel than the whole call: rounding
+                assert float((a - b.cpu()).abs().max()) <= 1e-13 * float(b.abs().max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [5000, 16383])
+def test_small_calls_need_no_scratch(n):
+    """Below the documented size a call runs without scratch, with too little or at an
+    unaligned address; the order of the points changes no bit."""
+    import torch
+    from agama_gpu_b200 import _lib
+    from agama_gpu_b200.synthetic import hernquist_points
+    pot = _multipole(32, nodes=100)
+    x = torch.from_numpy(hernquist_points(n, 10.0, 5)).cuda()
+    cargs = pot._c_args(0.0, x.device)
+    need = _lib.lib.agb_eval_scratch_bytes(*cargs, n, _lib.MODE_GRAD, 0)
+    ws = torch.empty(_lib.lib.agb_eval_workspace_bytes(*cargs, n, 0), dtype=torch.uint8, device="cuda")
+    if n == 16383:
+        assert 0 < need < ws.numel()
+    out = []
+    for p, room in ((ws.data_ptr(), ws.numel()), (None, 0), (ws.data_ptr(), 256), (ws.data_ptr() + 8, ws.numel() - 8)):
+        F = torch.empty_like(x)
+        assert _lib.lib.agb_eval_ws(*cargs, x.data_ptr(), n, _lib.MODE_GRAD, 0, None, F.data_ptr(),
+                                    None, None, 0, p, room, None) == 0
+        out.append(F)
+    F = torch.empty_like(x)
+    assert _lib.lib.agb_eval(*cargs, x.data_ptr(), n, _lib.MODE_GRAD, 0, None, F.data_ptr(), None,
+                             None, 0, None) == 0
+    torch.cuda.synchronize()
+    assert all(torch.equal(out[0], f) for f in out[1:] + [F])
+    # asked for by flag, the sort needs its scratch as before
+    assert _lib.lib.agb_eval_ws(*cargs, x.data_ptr(), n, _lib.MODE_GRAD, 0, None, F.data_ptr(), None,
+                                None, _lib.OUT_BIN_ALWAYS, None, 0, None) == -1
