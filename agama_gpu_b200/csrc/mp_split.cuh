@@ -5,14 +5,14 @@
 // with a chain of 289 steps at lmax 32.  Here a block takes a tile of at most 32 points
 // (lane = point) and its warps share the |m| groups; all lanes of a warp walk the same (l, m),
 // so there is no divergence and the recurrence constants stay uniform.  A group's sums are
-// formed by the operations of mp_harmonics_reg; the groups are added up slice by slice in
-// FP64 and one warp adds the slices' sums and finishes the leaf (with Hessians the groups are
-// kept apart and added in their order).  Consecutive leaves take turns between two buffers and
-// between finishing warps, so a leaf is finished while the next one is walked.
+// formed by the operations of mp_harmonics_reg and one warp adds the groups in their order and
+// finishes the leaf, so a point's result is that of one thread per point, bit for bit.
+// Consecutive leaves take turns between two buffers and between finishing warps, so a leaf is
+// finished while the next one is walked.
 #pragma once
 #include "multipole.cuh"
 
-// sums of a point that each slice adds up
+// sums of a point that each group adds to
 __host__ __device__ constexpr int split_sums(int mode) { return mode == AGB_MODE_POT ? 1 : 4; }
 // and, with Hessians, the values kept per |m| group: six of each trig column
 #define AGB_SPLIT_HESS_COLS 12
@@ -51,7 +51,7 @@ __device__ __forceinline__ void mp_group(const R* rec, int m, int lmax, R s, dou
     R sp[6];
     sp[0] = R(1); sp[1] = s; sp[2] = s * s; sp[3] = sp[2] * s; sp[4] = sp[2] * sp[2]; sp[5] = sp[4] * s;
     const R cth = (R)cth_d, sth = (R)sth_d;
-    const R c2 = (R)(cth_d * cth_d), w2 = (R)(-2.0 * cth_d * sth_d);
+    const R c2 = (R)__dmul_rn(cth_d, cth_d), w2 = (R)(-2.0 * cth_d * sth_d);
     int l0 = (PAR == 2) ? (m + (m & 1)) : m;
     if (m == 0) l0 = PAR;
     gc.zero();
@@ -130,19 +130,15 @@ __device__ __forceinline__ void mp_each_sum(MPSums& t, F f)
     if (MODE == AGB_MODE_GRAD) { f(2, t.Th); f(3, t.Pos); }
 }
 
-// The |m| groups are dealt out to `slices` in snake order: slice v of V takes m = p V + v on
-// even passes p and p V + V-1-v on odd ones, which gives every slice about the same number of
-// (l, m) steps.  A warp takes the slices w, w + S, ...  The slices depend on lmax alone, so a
-// point's sums do not depend on the number of warps.
-__host__ __device__ constexpr int split_slices(int lmax) { return lmax / 2 + 1 < 16 ? lmax / 2 + 1 : 16; }
-
-// The sums over slice v's groups, added up in FP64 (tot); with Hessians, where the order of
-// the groups shows (see mp_combine_hess), each group's columns are kept in cols
-// [m][value][point] for mp_split_hess.
+// The |m| groups are dealt out to the block's S warps in snake order: warp w takes m = p S + w
+// on even passes p and p S + S-1-w on odd ones, which gives every warp about the same number
+// of (l, m) steps.  What a group adds to each of the point's sums (with Hessians its columns,
+// see mp_combine_hess) is kept in out [m][value][point] and added up in ascending m, as
+// mp_harmonics_reg adds it: the same bits as one thread per point, whatever S is.
 template <int MODE, typename R, int PAR>
 __device__ __forceinline__ void mp_split_walk(const DevComp& c, int k, double s, double cth_d,
-                                              double sth_d, double cph, double sph, int v, int V,
-                                              MPSums& tot, R* cols, int T)
+                                              double sth_d, double cph, double sph, int w, int S,
+                                              void* out, int T)
 {
     constexpr bool HESS = MODE == AGB_MODE_HESS;
     const bool near_pole = sth_d < 1.0e-10;
@@ -150,8 +146,8 @@ __device__ __forceinline__ void mp_split_walk(const DevComp& c, int k, double s,
     const int lmax = c.lmax;
     double cm = 1.0, sm = 0.0, sinpow = 1.0, sinpow_m1 = 0.0;
     int at = 0;
-    for (int p = 0; p * V <= lmax; ++p) {
-        const int m = p * V + ((p & 1) ? V - 1 - v : v);
+    for (int p = 0; p * S <= lmax; ++p) {
+        const int m = p * S + ((p & 1) ? S - 1 - w : w);
         if (m > lmax) continue;
         for (; at < m; ++at) {
             if (!HESS) mp_rotate(cm, sm, cph, sph);
@@ -162,7 +158,7 @@ __device__ __forceinline__ void mp_split_walk(const DevComp& c, int k, double s,
         mp_group<MODE, R, PAR>(MPPtr<R>::base(c, k) + mp_group_start<PAR>(m, lmax) * MPPtr<R>::REC,
                                m, lmax, (R)s, cth_d, sth_d, sinpow, sinpow_m1, gc, gs);
         if (HESS) {
-            R* o = cols + (long long)m * AGB_SPLIT_HESS_COLS * T;
+            R* o = static_cast<R*>(out) + m * AGB_SPLIT_HESS_COLS * T;
             auto put = [&](int q, R a, R b) { o[2 * q * T] = a; o[(2 * q + 1) * T] = b; };
             put(0, gc.V, gs.V);
             put(1, gc.VR, gs.VR);
@@ -175,18 +171,21 @@ __device__ __forceinline__ void mp_split_walk(const DevComp& c, int k, double s,
         const R q1 = (near_pole && m == 1) ? R(1) : R(0);
         mp_col_finish<MODE, R>(gc, inv_sth, q1, R(0), R(0), R(0));
         mp_col_finish<MODE, R>(gs, inv_sth, q1, R(0), R(0), R(0));
-        const double md = (double)m;
-        tot.A += (double)gc.V * cm + (double)gs.V * sm;
-        if (MODE != AGB_MODE_POT) tot.B += (double)gc.VR * cm + (double)gs.VR * sm;
-        if (MODE == AGB_MODE_DENS) {
-            tot.D += (double)gc.VRR * cm + (double)gs.VRR * sm;
-            tot.L += (double)gc.L * cm + (double)gs.L * sm;
-        }
-        if (MODE == AGB_MODE_GRAD) {
-            tot.Th += (double)gc.VT * cm + (double)gs.VT * sm;
-            tot.Pos += md * ((double)gs.VP * cm - (double)gc.VP * sm);
-        }
+        MPSums t = {};
+        mp_combine<MODE, R>(t, gc, gs, m, cm, sm);
+        double* o = static_cast<double*>(out) + m * split_sums(MODE) * T;
+        mp_each_sum<MODE>(t, [&](int q, double& u) { o[q * T] = u; });
     }
+}
+
+// the sums of a point from its groups' shares, in ascending m
+template <int MODE>
+__device__ __forceinline__ void mp_split_total(int lmax, const double* shares, int T, MPSums& t)
+{
+    constexpr int NS = split_sums(MODE);
+    #pragma unroll 4
+    for (int m = 0; m <= lmax; ++m)
+        mp_each_sum<MODE>(t, [&](int q, double& u) { u += shares[(m * NS + q) * T]; });
 }
 
 // the groups of a Hessian leaf in ascending m, as mp_harmonics_reg adds them
@@ -235,38 +234,4 @@ __device__ __forceinline__ bool mp_place(const DevComp& c, double r, int& k, dou
     s = (logr - (logr_min + k * dlogr)) * inv_dlogr;
     s = fmin(fmax(s, 0.0), 1.0);
     return true;
-}
-
-// the end of multipole_point: the monopole, the log-scaling factor and the conversion
-template <int MODE>
-__device__ __forceinline__ void mp_close(const DevComp& c, int k, double s, const MPSums& t,
-                                         double px, double py, double pz, double inv_r, double Rc,
-                                         double cth, double sth, double cph, double sph,
-                                         PointOut& o)
-{
-    const double inv_dlogr = c.p[2], invPhi0 = c.p[3];
-    const double MP0 = AGB_MUL0 * AGB_PREFACT[0];
-    double c0, c0s, c0ss;
-    mp_quintic0(c, k, s, c0, c0s, c0ss);
-    if constexpr (MODE == AGB_MODE_HESS) {
-        mp_hess_end(t, inv_dlogr, invPhi0, c.log_scaling, c0, c0s, c0ss, px, py, pz, inv_r, Rc,
-                    cth, sth, cph, sph, o);
-        return;
-    }
-    const double dc0 = c0s * inv_dlogr;
-    const double d2c0 = c0ss * inv_dlogr * inv_dlogr;
-    double F = 1.0, dF = 0.0, d2F = 0.0, mono, dmono, d2mono;
-    if (c.log_scaling) {
-        const double ex = exp(c0);
-        const double P0 = 1.0 / (invPhi0 - ex);
-        const double dPdX = P0 * P0 * ex;
-        F = P0;
-        dF = dPdX * dc0;
-        d2F = dPdX * (d2c0 + dc0 * dc0 * P0 * (invPhi0 + ex));
-        mono = MP0 * F; dmono = MP0 * dF; d2mono = MP0 * d2F;
-    } else {
-        mono = MP0 * c0; dmono = MP0 * dc0; d2mono = MP0 * d2c0;
-    }
-    mp_finish<MODE>(t, inv_dlogr, F, dF, d2F, mono, dmono, d2mono, px, py, pz, inv_r, Rc,
-                    cth, sth, cph, sph, o);
 }

@@ -403,9 +403,10 @@ __device__ __forceinline__ void mp_col_finish(MPCol<R>& g, R inv_sth, R q1, R np
 }
 
 // One |m| group's sums combined with cos/sin(m phi), and the rotation to the next m, with
-// their roundings spelled out.  The Hessian walks use them (and mp_hess_end below): a
-// Hessian near the pole cancels terms of 1/sin(theta)^2, so kernels that are to agree in it
-// (one thread per point, batches, a block per tile) must round alike.
+// their roundings spelled out (as in mp_hess_end below), so that the kernels that add the
+// groups (one thread per point, batches, a block per tile) round alike: a point's result does
+// not depend on the kernel that a call takes, and a Hessian near the pole, which cancels
+// terms of 1/sin(theta)^2, shows every difference.
 __device__ __forceinline__ void mp_rotate(double& cm, double& sm, double cph, double sph)
 {
     const double t = fma(cm, cph, -__dmul_rn(sm, sph));
@@ -435,6 +436,27 @@ __device__ __forceinline__ void mp_combine_hess(MPSums& t, const MPCol<R>& gc, c
     add(t.ThPh, gc.VT, gs.VT, dTc, dTs);
 }
 
+// The same for the other modes' sums.
+template <int MODE, typename R>
+__device__ __forceinline__ void mp_combine(MPSums& t, const MPCol<R>& gc, const MPCol<R>& gs,
+                                           int m, double cm, double sm)
+{
+    auto add = [](double& s, R c, R v, double tc, double ts) {
+        s = __dadd_rn(s, fma((double)v, ts, __dmul_rn((double)c, tc)));
+    };
+    add(t.A, gc.V, gs.V, cm, sm);
+    if (MODE != AGB_MODE_POT) add(t.B, gc.VR, gs.VR, cm, sm);
+    if (MODE == AGB_MODE_DENS) {
+        add(t.D, gc.VRR, gs.VRR, cm, sm);
+        add(t.L, gc.L, gs.L, cm, sm);
+    }
+    if (MODE == AGB_MODE_GRAD) {
+        const double md = (double)m;
+        add(t.Th, gc.VT, gs.VT, cm, sm);
+        add(t.Pos, gc.VP, gs.VP, -md * sm, md * cm);
+    }
+}
+
 // GEN: the interval's records come from `slab` (this interval's row of a staged
 // copy of the FP32 table, possibly in shared memory) instead of the table itself
 template <int MODE, typename R, int PAR, bool GEN = false>
@@ -449,7 +471,7 @@ __device__ __forceinline__ void mp_harmonics_reg(const DevComp& c, int k, double
     R sp[6];
     sp[0] = R(1); sp[1] = s; sp[2] = s * s; sp[3] = sp[2] * s; sp[4] = sp[2] * sp[2]; sp[5] = sp[4] * s;
     const R cth = (R)cth_d, sth = (R)sth_d;
-    const R c2 = (R)(cth_d * cth_d), w2 = (R)(-2.0 * cth_d * sth_d);   // two-step walk
+    const R c2 = (R)__dmul_rn(cth_d, cth_d), w2 = (R)(-2.0 * cth_d * sth_d);   // two-step walk
     const R inv_sth = near_pole ? R(0) : (R)(1.0 / sth_d);
     const R cot = near_pole ? R(0) : (R)(cth_d / sth_d);
     const R np1 = near_pole ? R(0) : R(1);
@@ -460,13 +482,7 @@ __device__ __forceinline__ void mp_harmonics_reg(const DevComp& c, int k, double
     double cm = 1.0, sm = 0.0, sinpow = 1.0, sinpow_m1 = 0.0;
     for (int m = 0; m <= lmax; ++m) {
         if (m > 0) {
-            if constexpr (MODE == AGB_MODE_HESS) {
-                mp_rotate(cm, sm, cph, sph);
-            } else {
-                const double t = cm * cph - sm * sph;
-                sm = sm * cph + cm * sph;
-                cm = t;
-            }
+            mp_rotate(cm, sm, cph, sph);
             sinpow_m1 = sinpow;
             sinpow *= sth_d;
         }
@@ -551,18 +567,7 @@ __device__ __forceinline__ void mp_harmonics_reg(const DevComp& c, int k, double
             mp_combine_hess<R>(tot, gc, gs, m, cm, sm);
             continue;
         }
-        // combine the group's cos and sin sums with cos/sin(m phi) in FP64
-        const double md = (double)m;
-        const double dTc = -md * sm, dTs = md * cm;
-        tot.A += (double)gc.V * cm + (double)gs.V * sm;
-        if (MODE != AGB_MODE_POT) tot.B += (double)gc.VR * cm + (double)gs.VR * sm;
-        if (MODE == AGB_MODE_DENS)
-            tot.D += (double)gc.VRR * cm + (double)gs.VRR * sm;
-        if (MODE == AGB_MODE_DENS) tot.L += (double)gc.L * cm + (double)gs.L * sm;
-        if (NEED_ANG) {
-            tot.Th += (double)gc.VT * cm + (double)gs.VT * sm;
-            tot.Pos += (double)gc.VP * dTc + (double)gs.VP * dTs;
-        }
+        mp_combine<MODE, R>(tot, gc, gs, m, cm, sm);
     }
 }
 
@@ -577,13 +582,12 @@ __device__ __forceinline__ void mp_harmonics_reg2(const DevComp& c1, const DevCo
                                                   MPSums& tot2)
 {
     constexpr bool NEED_ANG = MODE == AGB_MODE_GRAD || MODE == AGB_MODE_HESS;
-    constexpr bool NEED_ANG2 = MODE == AGB_MODE_HESS;
     const bool near_pole = sth_d < 1.0e-10;
     const R s = (R)s_d;
     R sp[6];
     sp[0] = R(1); sp[1] = s; sp[2] = s * s; sp[3] = sp[2] * s; sp[4] = sp[2] * sp[2]; sp[5] = sp[4] * s;
     const R cth = (R)cth_d, sth = (R)sth_d;
-    const R cc2 = (R)(cth_d * cth_d), w2 = (R)(-2.0 * cth_d * sth_d);
+    const R cc2 = (R)__dmul_rn(cth_d, cth_d), w2 = (R)(-2.0 * cth_d * sth_d);
     const R inv_sth = near_pole ? R(0) : (R)(1.0 / sth_d);
     const R cot = near_pole ? R(0) : (R)(cth_d / sth_d);
     const R np1 = near_pole ? R(0) : R(1);
@@ -594,9 +598,7 @@ __device__ __forceinline__ void mp_harmonics_reg2(const DevComp& c1, const DevCo
     double cm = 1.0, sm = 0.0, sinpow = 1.0, sinpow_m1 = 0.0;
     for (int m = 0; m <= lmax; ++m) {
         if (m > 0) {
-            const double t = cm * cph - sm * sph;
-            sm = sm * cph + cm * sph;
-            cm = t;
+            mp_rotate(cm, sm, cph, sph);
             sinpow_m1 = sinpow;
             sinpow *= sth_d;
         }
@@ -679,28 +681,11 @@ __device__ __forceinline__ void mp_harmonics_reg2(const DevComp& c1, const DevCo
         };
         if (m == 0) walk(std::false_type());
         else walk(std::true_type());
-        const double md = (double)m;
-        const double dTc = -md * sm, dTs = md * cm;
         auto combine = [&](MPSums& tot, MPCol<R>& gc, MPCol<R>& gs) {
             mp_col_finish<MODE, R>(gc, inv_sth, q1, np1, cot, m2);
             mp_col_finish<MODE, R>(gs, inv_sth, q1, np1, cot, m2);
-            tot.A += (double)gc.V * cm + (double)gs.V * sm;
-            if (MODE != AGB_MODE_POT) tot.B += (double)gc.VR * cm + (double)gs.VR * sm;
-            if (MODE == AGB_MODE_HESS || MODE == AGB_MODE_DENS)
-                tot.D += (double)gc.VRR * cm + (double)gs.VRR * sm;
-            if (MODE == AGB_MODE_DENS) tot.L += (double)gc.L * cm + (double)gs.L * sm;
-            if (NEED_ANG) {
-                tot.Th += (double)gc.VT * cm + (double)gs.VT * sm;
-                tot.Pos += (double)gc.VP * dTc + (double)gs.VP * dTs;
-            }
-            if (NEED_ANG2) {
-                tot.Thth += (double)gc.VTT * cm + (double)gs.VTT * sm;
-                tot.BTh += (double)gc.VRT * cm + (double)gs.VRT * sm;
-                tot.Ph += (double)gc.V * dTc + (double)gs.V * dTs;
-                tot.Phph += -md * md * ((double)gc.V * cm + (double)gs.V * sm);
-                tot.BPh += (double)gc.VR * dTc + (double)gs.VR * dTs;
-                tot.ThPh += (double)gc.VT * dTc + (double)gs.VT * dTs;
-            }
+            if constexpr (MODE == AGB_MODE_HESS) mp_combine_hess<R>(tot, gc, gs, m, cm, sm);
+            else mp_combine<MODE, R>(tot, gc, gs, m, cm, sm);
         };
         combine(tot1, gc1, gs1);
         combine(tot2, gc2, gs2);
@@ -751,10 +736,11 @@ __device__ __forceinline__ void mp_finish(const MPSums& t, double inv_dlogr, dou
 {
     const double Bp = t.B * inv_dlogr;
     const double Dp = t.D * inv_dlogr * inv_dlogr;
-    o.phi = mono + F * t.A;
+    // roundings spelled out, as in mp_combine
+    o.phi = fma(F, t.A, mono);
     if (MODE == AGB_MODE_POT) return;
 
-    const double Pr = dmono + F * Bp + dF * t.A;
+    const double Pr = fma(dF, t.A, fma(F, Bp, dmono));
     if (MODE == AGB_MODE_DENS) {
         const double inv_r2 = inv_r * inv_r;
         const double lap = (d2mono + dmono) * inv_r2
@@ -765,9 +751,10 @@ __device__ __forceinline__ void mp_finish(const MPSums& t, double inv_dlogr, dou
     const double Pth = F * t.Th;
     const double Pos = F * t.Pos;
     const double inv_r2 = inv_r * inv_r;
-    o.g[0] = Pr * (px * inv_r2) + Pth * (cth * cph * inv_r) + Pos * (-sph * inv_r);
-    o.g[1] = Pr * (py * inv_r2) + Pth * (cth * sph * inv_r) + Pos * (cph * inv_r);
-    o.g[2] = Pr * (pz * inv_r2) + Pth * (-sth * inv_r);
+    auto two = [](double a, double b, double c, double d) { return fma(c, d, __dmul_rn(a, b)); };
+    o.g[0] = fma(Pos, -sph * inv_r, two(Pr, px * inv_r2, Pth, cth * cph * inv_r));
+    o.g[1] = fma(Pos, cph * inv_r, two(Pr, py * inv_r2, Pth, cth * sph * inv_r));
+    o.g[2] = two(Pr, pz * inv_r2, Pth, -sth * inv_r);
     if (MODE != AGB_MODE_HESS) return;
 
     // second derivatives in (log r, theta, phi)
@@ -914,6 +901,41 @@ __device__ __forceinline__ void mp_hess_end(const MPSums& t, double inv_dlogr, d
     }
 }
 
+// The end of a point inside the grid: the monopole (FP64), the log-scaling factor F(log r) with
+// its derivatives and the conversion.
+template <int MODE>
+__device__ __forceinline__ void mp_close(const DevComp& c, int k, double s, const MPSums& t,
+                                         double px, double py, double pz, double inv_r, double Rc,
+                                         double cth, double sth, double cph, double sph,
+                                         PointOut& o)
+{
+    const double inv_dlogr = c.p[2], invPhi0 = c.p[3];
+    const double MP0 = AGB_MUL0 * AGB_PREFACT[0];
+    double c0, c0s, c0ss;
+    mp_quintic0(c, k, s, c0, c0s, c0ss);
+    if constexpr (MODE == AGB_MODE_HESS) {
+        mp_hess_end(t, inv_dlogr, invPhi0, c.log_scaling, c0, c0s, c0ss, px, py, pz, inv_r, Rc,
+                    cth, sth, cph, sph, o);
+        return;
+    }
+    const double dc0 = c0s * inv_dlogr;
+    const double d2c0 = c0ss * inv_dlogr * inv_dlogr;
+    double F = 1.0, dF = 0.0, d2F = 0.0, mono, dmono, d2mono;
+    if (c.log_scaling) {
+        const double ex = exp(c0);
+        const double P0 = 1.0 / (invPhi0 - ex);
+        const double dPdX = P0 * P0 * ex;
+        F = P0;
+        dF = dPdX * dc0;
+        d2F = dPdX * (d2c0 + dc0 * dc0 * P0 * (invPhi0 + ex));
+        mono = MP0 * F; dmono = MP0 * dF; d2mono = MP0 * d2F;
+    } else {
+        mono = MP0 * c0; dmono = MP0 * dc0; d2mono = MP0 * d2c0;
+    }
+    mp_finish<MODE>(t, inv_dlogr, F, dF, d2F, mono, dmono, d2mono, px, py, pz, inv_r, Rc,
+                    cth, sth, cph, sph, o);
+}
+
 // STAGED: the records of intervals [k0, k1] are also in `slab` (a staged copy of
 // those rows of the FP32 table, in shared memory): a point in that range reads them
 // there (FP32 walks of regular structures; other points read the table)
@@ -923,7 +945,7 @@ __device__ __forceinline__ void multipole_point(const DevComp& c, double px, dou
                                                 const float* slab = nullptr, int k0 = 0,
                                                 int k1 = -1)
 {
-    const double logr_min = c.p[0], dlogr = c.p[1], inv_dlogr = c.p[2], invPhi0 = c.p[3];
+    const double logr_min = c.p[0], dlogr = c.p[1], inv_dlogr = c.p[2];
     const double in_s = c.p[4], in_U = c.p[5], in_W = c.p[6];
     const double out_s = c.p[7], out_U = c.p[8], out_W = c.p[9];
     const double MP0 = AGB_MUL0 * AGB_PREFACT[0];
@@ -997,32 +1019,8 @@ __device__ __forceinline__ void multipole_point(const DevComp& c, double px, dou
             mp_harmonics<MODE, R>(c, k, s, cth, sth, cph, sph, t);
     }
 
-    // monopole (FP64) and the log-scaling factor F(log r) with derivatives, after the
-    // walk so that its values are not live across it (FP64 kernel 7.22 -> 6.96 ms)
-    double c0, c0s, c0ss;
-    mp_quintic0(c, k, s, c0, c0s, c0ss);
-    if constexpr (MODE == AGB_MODE_HESS) {
-        mp_hess_end(t, inv_dlogr, invPhi0, c.log_scaling, c0, c0s, c0ss, px, py, pz, inv_r, Rc,
-                    cth, sth, cph, sph, o);
-        return;
-    }
-    const double dc0 = c0s * inv_dlogr;
-    const double d2c0 = c0ss * inv_dlogr * inv_dlogr;
-    double F = 1.0, dF = 0.0, d2F = 0.0, mono, dmono, d2mono;
-    if (c.log_scaling) {
-        const double ex = exp(c0);
-        const double P0 = 1.0 / (invPhi0 - ex);
-        const double dPdX = P0 * P0 * ex;
-        F = P0;
-        dF = dPdX * dc0;
-        d2F = dPdX * (d2c0 + dc0 * dc0 * P0 * (invPhi0 + ex));
-        mono = MP0 * F; dmono = MP0 * dF; d2mono = MP0 * d2F;
-    } else {
-        mono = MP0 * c0; dmono = MP0 * dc0; d2mono = MP0 * d2c0;
-    }
-
-    mp_finish<MODE>(t, inv_dlogr, F, dF, d2F, mono, dmono, d2mono, px, py, pz, inv_r, Rc,
-                    cth, sth, cph, sph, o);
+    // after the walk so that its values are not live across it (FP64 kernel 7.22 -> 6.96 ms)
+    mp_close<MODE>(c, k, s, t, px, py, pz, inv_r, Rc, cth, sth, cph, sph, o);
 }
 
 // Two Multipoles on one radial grid and column structure at the same point (the two
@@ -1035,7 +1033,6 @@ __device__ __forceinline__ void multipole_pair_point(const DevComp& c1, const De
                                                      PointOut& o1, PointOut& o2)
 {
     const double logr_min = c1.p[0], dlogr = c1.p[1], inv_dlogr = c1.p[2];
-    const double MP0 = AGB_MUL0 * AGB_PREFACT[0];
     const double r2 = px * px + py * py + pz * pz;
     const double r = sqrt(r2);
     const double logr = r < 1.0e-300 ? 0.0 : log(r);
@@ -1060,25 +1057,7 @@ __device__ __forceinline__ void multipole_pair_point(const DevComp& c1, const De
     else
         mp_harmonics_reg2<MODE, R, 1>(c1, c2, k, s, cth, sth, cph, sph, t1, t2);
     auto finish = [&](const DevComp& c, const MPSums& t, PointOut& o) {
-        const double invPhi0 = c.p[3];
-        double c0, c0s, c0ss;
-        mp_quintic0(c, k, s, c0, c0s, c0ss);
-        const double dc0 = c0s * inv_dlogr;
-        const double d2c0 = c0ss * inv_dlogr * inv_dlogr;
-        double F = 1.0, dF = 0.0, d2F = 0.0, mono, dmono, d2mono;
-        if (c.log_scaling) {
-            const double ex = exp(c0);
-            const double P0 = 1.0 / (invPhi0 - ex);
-            const double dPdX = P0 * P0 * ex;
-            F = P0;
-            dF = dPdX * dc0;
-            d2F = dPdX * (d2c0 + dc0 * dc0 * P0 * (invPhi0 + ex));
-            mono = MP0 * F; dmono = MP0 * dF; d2mono = MP0 * d2F;
-        } else {
-            mono = MP0 * c0; dmono = MP0 * dc0; d2mono = MP0 * d2c0;
-        }
-        mp_finish<MODE>(t, inv_dlogr, F, dF, d2F, mono, dmono, d2mono, px, py, pz, inv_r, Rc,
-                        cth, sth, cph, sph, o);
+        mp_close<MODE>(c, k, s, t, px, py, pz, inv_r, Rc, cth, sth, cph, sph, o);
     };
     finish(c1, t1, o1);
     finish(c2, t2, o2);

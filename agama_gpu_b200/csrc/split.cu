@@ -6,15 +6,15 @@
 // A few points per block, the harmonics split over its warps (mp_split.cuh): calls too small
 // to fill the GPU with one thread per point.  Block b evaluates the tile of a.chunk <= 32
 // points from b * a.chunk on.  Dynamic shared memory: two buffers of a.split_buf bytes with the
-// slices' sums [slice][sum][point] (Hessians: the groups' columns [m][value][point]), then every
-// leaf's results [leaf][value][point].
+// |m| groups' shares of the sums [m][sum][point] (Hessians: their columns), then every leaf's
+// results [leaf][value][point].
 template <int MODE, typename R, bool DYN>
 __global__ void __launch_bounds__(split_threads(MODE), 1)
 agb_split_kernel(const __grid_constant__ EvalArgs a)
 {
     constexpr bool VJP = MODE == AGB_MODE_VJP || MODE == AGB_MODE_VJPF;
     constexpr int CM = VJP ? AGB_MODE_HESS : MODE;
-    constexpr int NS = split_sums(CM), NO = split_out(CM);
+    constexpr int NO = split_out(CM);
     constexpr bool HESS = CM == AGB_MODE_HESS;
     extern __shared__ __align__(16) char split_smem[];
     __shared__ DevLeaf dyn_leaves[DYN ? AGB_MAX_LEAVES : 1];
@@ -44,7 +44,6 @@ agb_split_kernel(const __grid_constant__ EvalArgs a)
         const double ly = lf.sigma * y - lf.g1;
         const double lz = lf.sigma * z - lf.g2;
         const bool walked = c.kind == AGB_KIND_MULTIPOLE && c.structure != AGB_STRUCT_LIST;
-        const int V = split_slices(c.lmax);
         bool mine, grid = false;
         int k = 0;
         double s = 0.0, inv_r = 0.0, Rc = 0.0, cth = 1.0, sth = 0.0, cph = 1.0, sph = 0.0;
@@ -62,15 +61,11 @@ agb_split_kernel(const __grid_constant__ EvalArgs a)
                     sth = Rc * inv_r;
                     cph = (Rc > 1.0e-300) ? lx / Rc : 1.0;
                     sph = (Rc > 1.0e-300) ? ly / Rc : 0.0;
-                    for (int v = w; v < V; v += S) {
-                        MPSums t = {};
-                        if (c.structure == AGB_STRUCT_EVEN)
-                            mp_split_walk<CM, R, 2>(c, k, s, cth, sth, cph, sph, v, V, t, cols, T);
-                        else
-                            mp_split_walk<CM, R, 1>(c, k, s, cth, sth, cph, sph, v, V, t, cols, T);
-                        if (!HESS)
-                            mp_each_sum<CM>(t, [&](int q, double& u) { sums[(v * NS + q) * T] = u; });
-                    }
+                    void* out = HESS ? (void*)cols : (void*)sums;
+                    if (c.structure == AGB_STRUCT_EVEN)
+                        mp_split_walk<CM, R, 2>(c, k, s, cth, sth, cph, sph, w, S, out, T);
+                    else
+                        mp_split_walk<CM, R, 1>(c, k, s, cth, sth, cph, sph, w, S, out, T);
                 }
             }
             __syncthreads();
@@ -94,8 +89,7 @@ agb_split_kernel(const __grid_constant__ EvalArgs a)
                 else
                     mp_split_hess<R, 1>(c.lmax, cth, sth, cph, sph, cols, T, t);
             } else {
-                for (int v = 0; v < V; ++v)
-                    mp_each_sum<CM>(t, [&](int q, double& u) { u += sums[(v * NS + q) * T]; });
+                mp_split_total<CM>(c.lmax, sums, T, t);
             }
             mp_close<CM>(c, k, s, t, lx, ly, lz, inv_r, Rc, cth, sth, cph, sph, o);
         } else {
@@ -177,8 +171,8 @@ static bool split_shape(EvalArgs& a, int& S, int& T, size_t& smem)
     if (a.out_flags & AGB_OUT_SHAPE_BITS) return false;        // the caller's launch shape
     const long long sms = num_sms();
     if (a.n > sms * 32 * 22) return false;
-    // the heaviest Multipole stands for the tree: device-time leaves, which may pick any of the
-    // components, and the same leaves given by the host get the same kernel and the same bits
+    // the heaviest Multipole stands for the tree (device-time leaves may pick any of the
+    // components)
     int lmax = 0;
     long long steps = 0;                // (l, |m|) pairs of its walk
     for (const DevComp& c : a.comps) {
@@ -190,9 +184,9 @@ static bool split_shape(EvalArgs& a, int& S, int& T, size_t& smem)
     if (lmax < 2) return false;
     T = (int)std::min<long long>(32, (a.n + sms - 1) / sms);
     const long long tiles = ((a.n + T - 1) / T + sms - 1) / sms;     // of an SM
-    const int V = split_slices(lmax);
-    a.split_buf = T * (CM == AGB_MODE_HESS ? (lmax + 1) * AGB_SPLIT_HESS_COLS * (int)sizeof(R)
-                                           : V * split_sums(CM) * (int)sizeof(double));
+    const int V = lmax / 2 + 1;
+    a.split_buf = T * (lmax + 1) * (CM == AGB_MODE_HESS ? AGB_SPLIT_HESS_COLS * (int)sizeof(R)
+                                                        : split_sums(CM) * (int)sizeof(double));
     a.split_buf = (a.split_buf + 15) & ~15;
     // tiles that fit an SM's shared memory, with the results of eight leaves
     const int fit = AGB_SPLIT_SMEM / (2 * a.split_buf + 8 * split_out(CM) * T * (int)sizeof(double));
