@@ -181,7 +181,7 @@ def _load():
     lib.agb_eval_scratch_bytes.restype = ctypes.c_size_t
     lib.agb_eval_scratch_bytes.argtypes = [
         ctypes.POINTER(AgbComponent), ctypes.c_int, ctypes.POINTER(AgbLeaf), ctypes.c_int,
-        ctypes.c_int64, ctypes.c_int, ctypes.c_int]
+        ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_int]
     lib.agb_eval_wave_points.restype = ctypes.c_int64
     lib.agb_eval_wave_points.argtypes = [
         ctypes.POINTER(AgbComponent), ctypes.c_int, ctypes.POINTER(AgbLeaf), ctypes.c_int,

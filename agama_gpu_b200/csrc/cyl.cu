@@ -139,15 +139,20 @@ agb_cyl_kernel(const __grid_constant__ EvalArgs a)
     }
 }
 
+// false where the general kernel is the better one: force calls that it holds in one wave of 16
+// warps an SM while most warps here make a second pass (71041 to 75776 points; 33 against 39 us
+// at 75776, 35 against 31 at 76000, 33 against 31 at 64000, where a quarter of the warps do)
 template <int MODE, bool DYN>
-static void launch_cyl(EvalArgs& a, cudaStream_t st)
+static bool launch_cyl(EvalArgs& a, cudaStream_t st)
 {
     static std::atomic<int> per_sm[AGB_MAX_DEVICES];
     const int occ = blocks_per_sm(per_sm, agb_cyl_kernel<MODE, DYN>, AGB_CYL_BLOCK);
     const long long want = (a.n + AGB_CYL_BLOCK - 1) / AGB_CYL_BLOCK, slots = (long long)num_sms() * occ;
+    if (MODE == AGB_MODE_GRAD && a.n > slots * (AGB_CYL_BLOCK + 32) && a.n <= num_sms() * 512LL) return false;
     const long long grid = want < slots ? want : slots;
     a.chunk = ((a.n + grid - 1) / grid + 31) / 32 * 32;
     agb_cyl_kernel<MODE, DYN><<<(int)((a.n + a.chunk - 1) / a.chunk), AGB_CYL_BLOCK, 0, st>>>(a);
+    return true;
 }
 
 // FP64 calls of trees of cell-major CylSplines and analytic leaves, points unsorted, the default
@@ -167,9 +172,9 @@ bool agb_launch_cyl(int mode, bool mixed, EvalArgs& a, cudaStream_t st)
     }
     if (!any) return false;
     switch (mode) {
-    case AGB_MODE_POT:  a.dleaves ? launch_cyl<AGB_MODE_POT, true>(a, st) : launch_cyl<AGB_MODE_POT, false>(a, st); return true;
-    case AGB_MODE_GRAD: a.dleaves ? launch_cyl<AGB_MODE_GRAD, true>(a, st) : launch_cyl<AGB_MODE_GRAD, false>(a, st); return true;
-    case AGB_MODE_HESS: a.dleaves ? launch_cyl<AGB_MODE_HESS, true>(a, st) : launch_cyl<AGB_MODE_HESS, false>(a, st); return true;
+    case AGB_MODE_POT:  return a.dleaves ? launch_cyl<AGB_MODE_POT, true>(a, st) : launch_cyl<AGB_MODE_POT, false>(a, st);
+    case AGB_MODE_GRAD: return a.dleaves ? launch_cyl<AGB_MODE_GRAD, true>(a, st) : launch_cyl<AGB_MODE_GRAD, false>(a, st);
+    case AGB_MODE_HESS: return a.dleaves ? launch_cyl<AGB_MODE_HESS, true>(a, st) : launch_cyl<AGB_MODE_HESS, false>(a, st);
     default: return false;
     }
 }

@@ -414,31 +414,41 @@ struct BinPlan {
     bool one;          // sorted by bin_small, in slices of AGB_BIN_SMALL points
 };
 
-// What a point gains (ns) when the walk of this Multipole reads its records as broadcasts
-// instead of one row per lane.  The lanes' rows lie n_lm records of 48 bytes apart: rows that
-// fall on the same 16 bytes of a 128-byte line queue up in L1, so it depends on how many
-// different offsets the stride gives (1 to 8).  Measured, FP64 forces of 1M-4M points, sorted
-// against unsorted without the sort's cost (ns; harmonics, offsets): 0.09 (28, 2), 0.03
-// (45, 8), 0.06 (49, 8), 0.58 (64, 1), 0.13 (66, 4), 0.11 (81, 8), 0.11 (91, 8), 1.06 (144, 1);
-// with tables larger than the L1s 0.27 (153, 8), 1.2 (561, 8).  Mixed precision gains about
-// two thirds, the potential alone nearly twice as much.
-static double sort_gain(const agb_component& c, int mode)
+// What a point gains (ns) from the sort in this component.  A Multipole's walk reads its
+// records as broadcasts instead of one row per lane.  The lanes' rows lie n_lm records of 48
+// bytes apart: rows that fall on the same 16 bytes of a 128-byte line queue up in L1, so it
+// depends on how many different offsets the stride gives (1 to 8).  Measured, FP64 forces of
+// 1M-4M points, sorted against unsorted without the sort's cost (ns; harmonics, offsets): 0.09
+// (28, 2), 0.03 (45, 8), 0.06 (49, 8), 0.58 (64, 1), 0.13 (66, 4), 0.11 (81, 8), 0.11 (91, 8),
+// 1.06 (144, 1); with tables larger than the L1s 0.27 (153, 8), 1.2 (561, 8).  The potential
+// alone gains nearly twice as much, mixed precision a little less.  Multipoles in other frames
+// gain too, since the points of one interval lie together there as well (eight of lmax 8, each
+// in its own frame, 400003 points: 691 -> 513 us), and so do CylSplines, whose cells a warp's
+// points then share more often (13 harmonics beside a lmax-8 Multipole, 400003 points: forces
+// 341 -> 272 us, mixed 294 -> 251).
+static double sort_gain(const agb_component& c, int mode, int precision)
 {
+    const bool hess = mode == AGB_MODE_HESS || mode == AGB_MODE_VJP || mode == AGB_MODE_VJPF;
+    if (c.kind == AGB_KIND_CYLSPLINE) return c.n_lm * (hess ? 0.027 : 0.008);
+    if (c.kind != AGB_KIND_MULTIPOLE) return 0.0;
     int offsets = 8;
     for (int q = 8; q > 1 && (c.n_lm * 48 / 16) % (16 / q) == 0; q >>= 1) offsets = q / 2;
     const double l2 = 48.0 * c.n_lm * c.n_int > 400e3 ? 0.8e-3 : 0.0;
-    return c.n_lm * (6.5e-3 / offsets + 0.5e-3 + l2) * (mode == AGB_MODE_POT ? 1.7 : 1.0);
+    return c.n_lm * (6.5e-3 / offsets + 0.5e-3 + l2) * (mode == AGB_MODE_POT ? 1.7 : 1.0) *
+           (precision == AGB_PREC_MIXED ? 0.8 : 1.0);
 }
 
 // Whether sorting n points pays: the sort and the gather of the outputs cost 13 us, or 5 us
-// in one launch (bin_small), and 0.06 ns a point (0.16 with Hessians); half of the 13 us are
-// gained back by the kernel's coalesced stores and warmer rows, so the line lies at 6 us.
-// E.g. FP64 forces, sorted / unsorted: lmax 8 44 / 32 us at 100k points; lmax 12 103 / 108 at
-// 300k; lmax 16 45 / 46 us at 40k, 75 / 90 at 100k, 1490 / 2365 at 4M.
+// in one slice of bin_small, and 0.06 ns a point (0.16 with Hessians); part of the 13 us is
+// gained back by the kernel's coalesced stores and warmer rows, so the line lies at 8 us.
+// E.g. FP64 forces, unsorted / sorted: lmax 8 33 / 42 us at 100003 points; lmax 32 120 / 86 at
+// 3000 with one thread per point, but 19 / 21 split over warps, 62 / 33 at 10007; Multipole of
+// lmax 8 and CylSpline of 13 harmonics 43 / 49 at 24000, 124 / 100 at 100003.  The gains and
+// both lines are fitted together with the rule of the split kernel, see split.cu.
 static bool sort_pays(double gain, int64_t n, bool small, int mode)
 {
     const double cost = mode == AGB_MODE_HESS ? 0.16 : 0.06;
-    return (double)n * (gain - cost) > (small ? 5000.0 : 6000.0);
+    return (double)n * (gain - cost) > (small ? 5000.0 : 8000.0);
 }
 
 static bool sortable(const agb_component& c)
@@ -448,7 +458,7 @@ static bool sortable(const agb_component& c)
 
 // eval: an evaluation in `mode` (else an adjoint or table gradient, whose sums need the order)
 static BinPlan plan_binning(const agb_component* comps, const agb_leaf* leaves, int n_leaves,
-                            int64_t n, int out_flags, int eval = 0, int mode = -1)
+                            int64_t n, int out_flags, int eval = 0, int mode = 0, int precision = 0)
 {
     BinPlan b;
     memset(&b, 0, sizeof(b));
@@ -467,13 +477,8 @@ static BinPlan plan_binning(const agb_component* comps, const agb_leaf* leaves, 
     // sums over an interval's points (adjoints, table gradients) want long runs: one slice
     b.one = n <= (eval ? AGB_BIN_SLICED : AGB_BIN_SMALL) && c.n_int + 2 <= AGB_BIN_SMALL_BINS;
     if (eval && !(out_flags & AGB_OUT_BIN_ALWAYS)) {
-        double gain = 0.0;            // of every Multipole in the keyed one's frame
-        for (int L = 0; L < n_leaves; ++L) {
-            const agb_component& q = comps[leaves[L].comp];
-            if (q.kind == AGB_KIND_MULTIPOLE && leaves[L].sigma == leaves[best].sigma &&
-                !memcmp(leaves[L].gamma, leaves[best].gamma, sizeof(leaves[L].gamma)))
-                gain += sort_gain(q, mode);
-        }
+        double gain = 0.0;
+        for (int L = 0; L < n_leaves; ++L) gain += sort_gain(comps[leaves[L].comp], mode, precision);
         if (!sort_pays(gain, n, b.one && n <= AGB_BIN_SMALL, mode)) return b;
     }
     b.on = true;
@@ -676,7 +681,7 @@ static int eval_impl(const agb_component* comps, int n_comps, const agb_leaf* le
     a.gphi = g_vjp_phi; a.gforce = g_vjp_force;
     if ((rc = pack_args(a, comps, n_comps, leaves, n_leaves, precision))) return rc;
 
-    BinPlan b = plan_binning(comps, leaves, n_leaves, n, out_flags, 1, mode);
+    BinPlan b = plan_binning(comps, leaves, n_leaves, n, out_flags, 1, mode, precision);
     if (sort_optional(n, out_flags) &&
         (own_ws || !workspace || ((uintptr_t)workspace & 255u) || workspace_bytes < ws_bytes(b, n)))
         b.on = false;
@@ -726,12 +731,12 @@ extern "C" size_t agb_eval_workspace_bytes(const agb_component* comps, int n_com
 
 extern "C" size_t agb_eval_scratch_bytes(const agb_component* comps, int n_comps,
                                          const agb_leaf* leaves, int n_leaves, int64_t n, int mode,
-                                         int out_flags)
+                                         int precision, int out_flags)
 {
     if (!comps || !leaves || n_leaves < 1 || n_comps < 1) return 0;
     for (int L = 0; L < n_leaves; ++L)
         if (leaves[L].comp < 0 || leaves[L].comp >= n_comps) return 0;
-    const BinPlan b = plan_binning(comps, leaves, n_leaves, n, out_flags, 1, mode);
+    const BinPlan b = plan_binning(comps, leaves, n_leaves, n, out_flags, 1, mode, precision);
     return b.one ? ws_bytes(b, n) : ws_bytes_staged(b, n);
 }
 
@@ -1099,6 +1104,10 @@ extern "C" int agb_eval_timed(const agb_component* comps, int n_comps, const agb
     for (int c = 0; c < n_comps; ++c)
         if ((rc = comp_to_dev(comps[c], a.comps[c], precision))) return rc;
     a.n_leaves = p->n;
+    for (int L = 0; L < p->n; ++L) {        // what the choice of the kernel looks at
+        a.leaves[L].comp = lv[L].comp;
+        a.leaves[L].ampl = 1.0;
+    }
     DevLeaf* dl = (DevLeaf*)workspace;
     a.dleaves = dl;
     int pair[AGB_MAX_LEAVES];
@@ -1106,7 +1115,7 @@ extern "C" int agb_eval_timed(const agb_component* comps, int n_comps, const agb
     if ((rc = launch_time_leaves(p, pair, step, t0, dt, off, dl, st))) return rc;
     char* ws = (char*)workspace + TP_LEAF_BYTES;
     const size_t room = workspace_bytes - TP_LEAF_BYTES;
-    BinPlan b = plan_binning(comps, lv, p->n, n, out_flags, 1, mode);
+    BinPlan b = plan_binning(comps, lv, p->n, n, out_flags, 1, mode, precision);
     if (sort_optional(n, out_flags) && room < ws_bytes(b, n)) b.on = false;
     if (b.on) {
         b.key.leaf = dl + b.leaf;

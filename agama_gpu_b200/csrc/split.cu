@@ -1,4 +1,5 @@
 // split.cu -- the kernel for calls too small to fill the GPU with one thread per point.
+#include <cmath>
 #include "eval_point.cuh"
 #include "launch.cuh"
 #include "mp_split.cuh"
@@ -136,73 +137,129 @@ agb_split_kernel(const __grid_constant__ EvalArgs a)
 }
 
 // dynamic shared memory of a block: lmax 32 with Hessians in FP64 needs 203 KB of columns, and
-// 10 KB per four leaves of results (larger trees take one thread per point there)
+// 2.5 KB per leaf of results (larger trees take one thread per point there)
 #define AGB_SPLIT_SMEM (220 * 1024)
 
-// Estimated time of an SM that evaluates `tiles` tiles with S warps each (S = 1: one thread
-// per point), `cap` tiles at a time: per wave of resident warps the steps of a warp, each as
-// long as the latency of one step (lat) or as the warps keep the pipe busy, and the tile's
-// finish, in units of one warp's pipe time per step.
-static long long split_cost(long long tiles, int S, long long cap, long long steps, int lat,
-                            int finish)
+// What a call's leaves cost a warp, in units of the latency of one (l, |m|) step.
+struct SplitWork {
+    double steps = 0.0;            // of the regular Multipoles, which the warps share
+    int walked = 0;                // how many of them
+    int groups = 0;                // and their |m| groups
+    int lmax = 0;                  // most of any component, in use or (device-time leaves) not yet
+    double columns = 0.0;          // of the other Multipoles,
+    double harmonics = 0.0;        // of the CylSplines: one warp each
+    int analytic = 0;
+};
+
+static SplitWork split_work(const EvalArgs& a)
 {
+    SplitWork t;
+    for (const DevComp& c : a.comps)
+        if (c.kind == AGB_KIND_MULTIPOLE && c.structure != AGB_STRUCT_LIST) t.lmax = std::max(t.lmax, c.lmax);
+    for (int L = 0; L < a.n_leaves; ++L) {
+        if (a.leaves[L].ampl == 0.0) continue;
+        const DevComp& c = a.comps[a.leaves[L].comp];
+        const int h = c.lmax / 2 + 1, l1 = c.lmax + 1;
+        if (c.kind == AGB_KIND_CYLSPLINE) {
+            t.harmonics += c.n_lm;
+        } else if (c.kind != AGB_KIND_MULTIPOLE) {
+            ++t.analytic;
+        } else if (c.structure == AGB_STRUCT_LIST) {
+            t.columns += c.n_lm;
+        } else {
+            ++t.walked;
+            t.groups += l1;
+            t.steps += c.structure == AGB_STRUCT_EVEN ? h * h : l1 * (l1 + 1) / 2;
+        }
+    }
+    return t;
+}
+
+// Constants of the estimate below, in the same unit (0.25-0.35 us in FP64, 0.17-0.25 mixed).
+struct SplitRates {
+    double pipe, rows;             // a step's pipe time with broadcast records, and with a row per
+                                   // lane (unsorted points, in proportion to the tile's lanes)
+    double finish, group;          // finishing a walked leaf: its end and barrier, and per group
+    double unsorted, mixed;        // factors of these: unsorted steps are longer, mixed ones shorter
+    double analytic, analytic_pipe;
+    double harmonic, harmonic_pipe;
+    double margin;                 // a split has to be better by this
+    double overlap;                // of the rounding up to whole waves, what tiles that end at
+                                   // different times save
+};
+
+// Estimated time of an SM that evaluates `tiles` tiles of T points with S warps each (S = 1:
+// one thread per point), `cap` tiles at a time: per wave of resident warps the steps of a warp,
+// whose latency and whose share of the pipe's time add in quadrature, the finish of each leaf,
+// and the other leaves, which the tile's warps take in turn.
+static double split_time(const SplitWork& t, const SplitRates& r, long long tiles, int T, int S,
+                         long long cap, bool sorted, bool mixed)
+{
+    const double pipe = sorted ? r.pipe : r.pipe + (r.rows - r.pipe) * T / 32;
+    auto hypot2 = [](double a, double b) { return std::sqrt(a * a + b * b); };
+    auto wave = [&](double k) {
+        double x = t.steps / S * hypot2(1.0, k * S * pipe);
+        if (S > 1)
+            x += (t.walked * r.finish + t.groups * r.group) * (sorted ? 1.0 : r.unsorted) * (mixed ? r.mixed : 1.0);
+        x += (double)t.analytic / S * hypot2(r.analytic, k * S * r.analytic_pipe);
+        x += t.harmonics * hypot2(r.harmonic, k * r.harmonic_pipe);
+        return x + t.columns * std::max(0.3, k * 0.06);
+    };
     const long long full = tiles / cap, rest = tiles % cap;
-    auto wave = [&](long long n) { return steps * std::max<long long>(lat, n * S) + finish; };
-    return full * wave(cap) + (rest ? wave(rest) : 0);
+    if (S == 1) return full * wave((double)cap) + (rest ? wave((double)rest) : 0.0);
+    const double exact = std::max(1.0, (double)tiles / cap), whole = (double)(full + (rest ? 1 : 0));
+    const double free = r.overlap * (1.0 - 1.0 / cap);
+    return wave((double)std::min(tiles, cap)) * (exact * free + whole * (1.0 - free)) * r.margin;
 }
 
 // The split kernel's shape for this call: S warps per tile of T points; false where one
 // thread per point is the better one (or the tree has no Multipole to split).
 //
-// T spreads the points over the SMs, at most 32 to a tile.  S comes from the estimate above:
-// an SM holds 16 warps at 128 registers (8 at 255, the Hessian modes), a step's latency is
-// about the pipe time of 11 warps (6), and finishing a leaf of a tile costs about 60 steps of
-// one warp (twice that with Hessians).
-// Measured (Multipole alone, FP64 force, one thread per point -> split): lmax 32 10k points
-// 119 -> 45 us (S = 5), 20k 119 -> 73 (S = 3), 40k 167 -> 138 (S = 3), 100k 331 -> 290
-// (S = 2), 300k 661 -> 768; lmax 16 40k 50 -> 46, 100k 96 -> 90; lmax 8 10k 15.5 -> 9.1,
-// 20k 15.7 -> 11.5; lmax 4 40k 9.9 -> 12.4; the galaxy tree (lmax 16) with Hessians at 1000
-// points 39 -> 11; the Milky Way tree (lmax 32) at 1000 points 187 -> 24.
+// T spreads the points over the SMs, at most 32 to a tile.  S comes from the estimate above,
+// with the warps that an SM holds (16 at 128 registers, 8 at 255 with Hessians) and the tiles
+// that fit its shared memory.  The rates are fitted to 26 trees (lmax 2 to 32, one to eight
+// Multipoles, regular or not, with CylSplines and up to 20 analytic leaves), up to 26 sizes from
+// 300 to 400003 points, four modes, both precisions, sorted and not, each with S = 1 to 16 (in
+// steps of a third or less): over those 4768 calls the shape taken is 2 % (geometric mean) from
+// the best one tried, and slower than one thread per point on points sorted from 16384 on by
+// more than 5 % in 31 (up to 22 %: 20 analytic leaves with Hessians).  Forces, one thread per
+// point -> split, us: lmax 8 FP64 1000 points 17 -> 9, 10007 17 -> 11, 24000 17 -> 15, 40009 20
+// (not split); lmax 32 FP64 10007 89 -> 33, 40009 100 -> 78, mixed 58 -> 29, 69 -> 64; lmax 16
+// with 20 analytic leaves, mixed, 100003 84 (not split; two warps a tile take 156).
 template <int MODE, typename R>
 static bool split_shape(EvalArgs& a, int& S, int& T, size_t& smem)
 {
     constexpr int CM = (MODE == AGB_MODE_VJP || MODE == AGB_MODE_VJPF) ? AGB_MODE_HESS : MODE;
+    constexpr bool HESS = CM == AGB_MODE_HESS;
+    constexpr bool mixed = std::is_same<R, float>::value;
     constexpr int warps = split_threads(MODE) / 32;
+    static constexpr SplitRates rates = HESS
+        ? SplitRates{0.06, 0.23, 4.0, 0.7, 0.38, 1.4, 0.66, 2.8, 1.35, 0.32, 1.068, 0.3}
+        : SplitRates{0.066, 0.1, 3.5, 0.35, 0.55, 1.5, 0.5, 1.2, 2.5, 0.36, 1.025, 0.5};
     if (a.out_flags & AGB_OUT_SHAPE_BITS) return false;        // the caller's launch shape
+    const SplitWork work = split_work(a);
+    if (work.lmax < 2 || !work.walked) return false;
     const long long sms = num_sms();
-    if (a.n > sms * 32 * 22) return false;
-    // the heaviest Multipole stands for the tree (device-time leaves may pick any of the
-    // components)
-    int lmax = 0;
-    long long steps = 0;                // (l, |m|) pairs of its walk
-    for (const DevComp& c : a.comps) {
-        if (c.kind != AGB_KIND_MULTIPOLE || c.structure == AGB_STRUCT_LIST) continue;
-        const long long h = c.lmax / 2 + 1, l1 = c.lmax + 1;
-        lmax = std::max(lmax, c.lmax);
-        steps = std::max(steps, c.structure == AGB_STRUCT_EVEN ? h * h : l1 * (l1 + 1) / 2);
-    }
-    if (lmax < 2) return false;
     T = (int)std::min<long long>(32, (a.n + sms - 1) / sms);
-    const long long tiles = ((a.n + T - 1) / T + sms - 1) / sms;     // of an SM
-    const int V = lmax / 2 + 1;
-    a.split_buf = T * (lmax + 1) * (CM == AGB_MODE_HESS ? AGB_SPLIT_HESS_COLS * (int)sizeof(R)
-                                                        : split_sums(CM) * (int)sizeof(double));
+    a.split_buf = T * (work.lmax + 1) * (HESS ? AGB_SPLIT_HESS_COLS * (int)sizeof(R)
+                                              : split_sums(CM) * (int)sizeof(double));
     a.split_buf = (a.split_buf + 15) & ~15;
-    // tiles that fit an SM's shared memory, with the results of eight leaves
-    const int fit = AGB_SPLIT_SMEM / (2 * a.split_buf + 8 * split_out(CM) * T * (int)sizeof(double));
-    const int lat = warps == 16 ? 11 : 6;
-    long long best = split_cost(tiles, S = 1, warps, steps, lat, 0);
-    for (int s = 2; s <= std::min(warps, V); ++s) {
-        const int cap = std::max(1, std::min(warps / s, fit));
-        const long long t = split_cost(tiles, s, cap, steps * ((V + s - 1) / s) / V, lat,
-                                       CM == AGB_MODE_HESS ? 120 : 60);
+    smem = 2 * (size_t)a.split_buf + sizeof(double) * T * (size_t)a.n_leaves * split_out(CM);
+    if (smem > AGB_SPLIT_SMEM) return false;
+    const int fit = std::max(1, 228 * 1024 / ((int)smem + 1024));
+    auto per_sm = [&](long long tile) { return ((a.n + tile - 1) / tile + sms - 1) / sms; };
+    const bool sorted = a.perm || a.stage;
+    double best = split_time(work, rates, per_sm(32), 32, S = 1, warps, sorted, mixed);
+    for (const int s : {2, 3, 4, 5, 6, 8, 11, 16}) {
+        if (s > std::min(warps, work.lmax / 2 + 1)) break;
+        const double t = split_time(work, rates, per_sm(T), T, s, std::max(1, std::min(warps / s, fit)),
+                                    sorted, mixed);
         if (t < best) {
             best = t;
             S = s;
         }
     }
-    smem = 2 * (size_t)a.split_buf + sizeof(double) * T * (size_t)a.n_leaves * split_out(CM);
-    return S >= 2 && smem <= AGB_SPLIT_SMEM;
+    return S >= 2;
 }
 
 template <int MODE, typename R, bool DYN>

@@ -433,8 +433,8 @@ class _GPUPotBase:
             f |= tuned.get((mode, prec, int(n).bit_length()), 0)
         return f
 
-    def _workspace(self, cargs, n: int, dev: torch.device, flags: int, mode: int):
-        nws = int(_lib.lib.agb_eval_scratch_bytes(*cargs, n, mode, flags))
+    def _workspace(self, cargs, n: int, dev: torch.device, flags: int, mode: int, prec: int):
+        nws = int(_lib.lib.agb_eval_scratch_bytes(*cargs, n, mode, prec, flags))
         return (torch.empty(nws, dtype=torch.uint8, device=dev) if nws else None), nws
 
     def _launch(self, arr: torch.Tensor, t: float, mode: int, want_phi: bool,
@@ -463,7 +463,7 @@ class _GPUPotBase:
         ptr = lambda a: None if a is None else a.data_ptr()  # noqa: E731
         stream = torch._C._cuda_getCurrentRawStream(dev.index)     # 0.1 us, a Stream object 2.2
         flags = self._flags(mode, prec, n)
-        ws, nws = self._workspace(cargs, n, dev, flags, mode)
+        ws, nws = self._workspace(cargs, n, dev, flags, mode, prec)
         rc = _lib.lib.agb_eval_ws(*cargs, arr.data_ptr(), n, mode, prec, ptr(phi), ptr(grad),
                                   ptr(hess), ptr(rho), flags, ptr(ws), nws,
                                   stream)
@@ -486,7 +486,8 @@ class _GPUPotBase:
         gp = None if g_phi is None else g_phi.to(device=dev, dtype=torch.float64).contiguous()
         gf = None if g_force is None else g_force.to(device=dev, dtype=torch.float64).contiguous()
         ptr = lambda a: None if a is None else a.data_ptr()  # noqa: E731
-        ws, nws = self._workspace(cargs, n, dev, 0, _lib.MODE_VJP)   # agb_eval_vjp sorts by default
+        # agb_eval_vjp sorts by default
+        ws, nws = self._workspace(cargs, n, dev, 0, _lib.MODE_VJP, prec)
         stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
         if force_out is None:
             rc = _lib.lib.agb_eval_vjp(*cargs, arr.data_ptr(), n, prec, ptr(gp), ptr(gf),
@@ -793,7 +794,8 @@ class _GPUPotBase:
         if cargs is None:
             cargs = self._c_args(t, dev)
         # the leaves at t decide which chunks sort
-        nws = max(int(_lib.lib.agb_eval_scratch_bytes(*cargs, m, mode, f)) for m, f in flags.items())
+        nws = max(int(_lib.lib.agb_eval_scratch_bytes(*cargs, m, mode, prec, f))
+                  for m, f in flags.items())
         ws = pipe["bufs"].get("ws")
         if nws and (ws is None or ws.numel() < nws):
             # allocated on the compute stream, the only one that uses it

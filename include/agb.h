@@ -69,7 +69,9 @@ extern "C" {
    (bounded) and reads global memory from then on: the results are those of the
    unstaged kernel */
 #define AGB_OUT_STAGE_GIVE_UP (1 << 24)
-/* Launch-shape knobs of the evaluation kernel.  Results do not depend on them;
+/* Launch-shape knobs of the evaluation kernel with one thread per point (with none of
+   them set the library takes another kernel where that is faster: small calls,
+   CylSplines).  Results do not depend on them, nor on how many points share a call;
    the autotuner (agama_gpu_b200/autotune.py) times them.  No counterpart in the
    reference, whose launch shape is fixed.
    bits 8-11:  blocks per resident slot of the grid, 1-15 (0: the default, one
@@ -239,7 +241,7 @@ size_t agb_eval_workspace_bytes(const agb_component* comps, int n_comps,
                                 int out_flags);
 size_t agb_eval_scratch_bytes(const agb_component* comps, int n_comps,
                               const agb_leaf* leaves, int n_leaves, int64_t n, int mode,
-                              int out_flags);
+                              int precision, int out_flags);
 int agb_eval_ws(const agb_component* comps, int n_comps,
                 const agb_leaf* leaves, int n_leaves,
                 const double* xyz, int64_t n, int mode, int precision,

@@ -32,10 +32,11 @@ def test_workspace_of_the_largest_call_serves_smaller_ones(lmax):
         most = b
         for args in (one, two):
             for mode in range(5):
-                for flags in (0, _lib.OUT_BIN_ALWAYS):
-                    assert _lib.lib.agb_eval_scratch_bytes(*args, n, mode, flags) <= most
+                for prec in (_lib.PREC_FP64, _lib.PREC_MIXED):
+                    for flags in (0, _lib.OUT_BIN_ALWAYS):
+                        assert _lib.lib.agb_eval_scratch_bytes(*args, n, mode, prec, flags) <= most
     assert _lib.lib.agb_eval_workspace_bytes(*two, 10**6, _lib.OUT_NO_BINNING) == 0
-    assert _lib.lib.agb_eval_scratch_bytes(*two, 10**6, _lib.MODE_POT, _lib.OUT_NO_BINNING) == 0
+    assert _lib.lib.agb_eval_scratch_bytes(*two, 10**6, _lib.MODE_POT, 0, _lib.OUT_NO_BINNING) == 0
 
 
 def _multipole(lmax, seed=3, nodes=50):
@@ -73,7 +74,7 @@ def test_small_calls_need_no_scratch(n):
     pot = _multipole(32, nodes=100)
     x = torch.from_numpy(hernquist_points(n, 10.0, 5)).cuda()
     cargs = pot._c_args(0.0, x.device)
-    need = _lib.lib.agb_eval_scratch_bytes(*cargs, n, _lib.MODE_GRAD, 0)
+    need = _lib.lib.agb_eval_scratch_bytes(*cargs, n, _lib.MODE_GRAD, 0, 0)
     ws = torch.empty(_lib.lib.agb_eval_workspace_bytes(*cargs, n, 0), dtype=torch.uint8, device="cuda")
     if n == 16383:
         assert 0 < need < ws.numel()
@@ -91,3 +92,58 @@ def test_small_calls_need_no_scratch(n):
     # asked for by flag, the sort needs its scratch as before
     assert _lib.lib.agb_eval_ws(*cargs, x.data_ptr(), n, _lib.MODE_GRAD, 0, None, F.data_ptr(), None,
                                 None, _lib.OUT_BIN_ALWAYS, None, 0, None) == -1
+
+
+def test_other_frames_and_cylsplines_count_for_the_sort():
+    """Sorting by one Multipole's intervals helps Multipoles in other frames and CylSplines."""
+    from agama_gpu_b200 import _lib
+    frames = _descriptors(45, n_leaves=8)
+    for i in range(8):
+        frames[2][i].gamma[0] = float(i)
+    barred = _descriptors(45, n_leaves=2)
+    barred[0][1].kind, barred[0][1].n_lm = _lib.KIND_CYLSPLINE, 13
+    alone = _descriptors(45)
+    for n in (100003, 400003):
+        for mode in (_lib.MODE_GRAD, _lib.MODE_HESS):
+            # 691 -> 513 us (forces) of the eight, 341 -> 272 with the CylSpline at 400003 points
+            assert _lib.lib.agb_eval_scratch_bytes(*frames, n, mode, _lib.PREC_FP64, 0) > 0
+            assert _lib.lib.agb_eval_scratch_bytes(*barred, n, mode, _lib.PREC_FP64, 0) > 0
+            # 62 -> 87 us: one small table is read from L1 in any order
+            assert _lib.lib.agb_eval_scratch_bytes(*alone, n, mode, _lib.PREC_FP64, 0) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tree,n,prec", [("analytic", 100003, "mixed"), ("four", 100003, "mixed"),
+                                         ("analytic", 40009, "fp64"), ("frames", 131072, "fp64")])
+def test_default_call_is_no_slower_than_one_thread_per_point(tree, n, prec):
+    """Trees with many leaves: the kernel that the rules pick against one thread per point on
+    sorted points (1.4 to 1.85 times as slow before the rules looked at all leaves)."""
+    import torch
+    import agama_gpu_b200 as agb
+    from agama_gpu_b200 import _lib
+    from agama_gpu_b200.synthetic import hernquist_points
+    shift = lambda p, i: agb.ShiftedPotentialGPU(p, [float(i), 1.0, 0.0])  # noqa: E731
+    leaves = {"analytic": lambda: [_multipole(16, nodes=64)] + [
+                  shift(agb.PlummerPotentialGPU(mass=1e9, scaleRadius=0.5), i) for i in range(20)],
+              "four": lambda: [_multipole(16, s, 64) for s in range(4)],
+              "frames": lambda: [shift(_multipole(8, 3, 64), i) for i in range(8)]}[tree]()
+    pot = agb.CompositePotentialGPU(leaves)
+    x = torch.from_numpy(hernquist_points(n, 10.0, 5)).cuda()
+    base = type(pot)._flags
+
+    def time(flags):
+        pot._flags = lambda *a: base(pot, *a) | flags
+        best = 1e9
+        for _ in range(8):
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record()
+            for _ in range(8):
+                pot._launch(x, 0.0, _lib.MODE_POT if tree == "frames" else _lib.MODE_GRAD, False,
+                            precision=prec)
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        del pot._flags
+        return best
+    time(0)
+    assert time(0) < 1.25 * time(_lib.OUT_BIN_ALWAYS | 2 << _lib.OUT_GRID_SHIFT)
