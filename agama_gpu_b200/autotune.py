@@ -13,10 +13,13 @@ harmonics, how many components), the number of points and the mode:
 * block size: 256, 128 or 512 threads (512 in the potential, force and
   density modes); the resident-block bound scales so every size keeps the
   same registers per thread.
-* binning: sort the points by radial interval first (default from
-  AGB_BIN_MIN_POINTS points on), never, or always.  The sort costs three small
-  launches and 32 B of scratch per point; it pays when the harmonic sums are
-  long.
+* no shape at all: the library's own choice, which for small calls shares the
+  harmonics over a block's warps and for FP64 CylSplines loads a warp's
+  records together (those kernels have no shapes to choose from).
+* binning: sort the points by radial interval first, or never (untuned calls
+  sort where an estimate says that it pays).  The sort costs one launch up to
+  131072 points, three beyond, and 32 B of scratch per point (112 with the
+  outputs in sorted order); it pays when the harmonic sums are long.
 * tile_points and stage (batches): points per work-queue tile of a
   BatchedPotentialGPU, and whether each tile's table rows are bulk-copied (TMA)
   into shared memory or read through L1/L2.
@@ -49,6 +52,10 @@ MODES = {"potential": _lib.MODE_POT, "force": _lib.MODE_GRAD, "forceDeriv": _lib
 GRIDS = (1, 2, 4, 8)
 PPTS = (1, 4, 16, 64)                   # points per thread (powers of two)
 BLOCKS = {256: 0, 128: 1, 512: 2}       # threads per block -> AGB_OUT_BLOCK code
+
+# version of the candidates, part of the cache key: a choice made among other candidates (the
+# shapes alone, without the library's own choice) is not applied
+CANDIDATES = 2
 
 _lock = threading.Lock()
 
@@ -83,8 +90,8 @@ def _store(key: str, value: dict) -> None:
 
 
 def signature(pot, mode: int, prec: int, n: int, t: float = 0.0) -> str:
-    """Cache key: GPU, leaves (kind, harmonics, intervals, structure), mode, precision,
-    and the size class of the call (bit length of the point count)."""
+    """Cache key: GPU, leaves (kind, harmonics, intervals, structure), mode, precision, the
+    size class of the call (bit length of the point count) and the candidates' version."""
     dev = torch.cuda.get_device_properties(torch.cuda.current_device())
     leaves = []
     for c, _, _, _ in pot._leaves(float(t)):
@@ -92,7 +99,7 @@ def signature(pot, mode: int, prec: int, n: int, t: float = 0.0) -> str:
         leaves.append((int(c.kind), int(getattr(c, "_n_cols", getattr(tb, "n_lm", 0)) or 0),
                        int(getattr(tb, "n_int", 0) or 0), int(getattr(c, "_structure", 0) or 0)))
     return json.dumps([dev.name, dev.multi_processor_count, sorted(leaves), mode, prec,
-                       int(n).bit_length()])
+                       int(n).bit_length(), CANDIDATES])
 
 
 def _time(fn, reps: int) -> float:
@@ -107,18 +114,31 @@ def _time(fn, reps: int) -> float:
     return e0.elapsed_time(e1) / reps
 
 
+def _default_shape(n: int, mode: int):
+    """(threads per block, schedule) that the one-thread-per-point kernel takes when no shape is
+    set, for a tree with a Multipole."""
+    if n <= 1 << 21:
+        return 256, "grid2"
+    return {_lib.MODE_POT: (256, "grid1"), _lib.MODE_HESS: (128, "grid1")}.get(mode, (512, "grid1"))
+
+
 def _candidates(n: int, mode: int = _lib.MODE_GRAD):
-    """(name, extra out_flags) pairs for a call of n points in this mode."""
+    """(name, extra out_flags) pairs for a call of n points in this mode.  In the place of the
+    shape that is the default one stands no shape: the library's own choice of kernel."""
     out = []
     bins = [("sort", _lib.OUT_BIN_ALWAYS), ("nosort", _lib.OUT_NO_BINNING)]
     scheds = [(f"grid{g}", g << _lib.OUT_GRID_SHIFT) for g in GRIDS]
     scheds += [(f"ppt{p}", (p.bit_length()) << _lib.OUT_PPT_SHIFT) for p in PPTS]
+    default = _default_shape(n, mode)
     for name, bf in bins:
         for bs, code in BLOCKS.items():
             if bs == 512 and mode == _lib.MODE_HESS:
                 continue                 # the Hessian kernel runs 256 threads at most
             for sname, sf in scheds:
-                out.append((f"{name}/b{bs}/{sname}", bf | (code << _lib.OUT_BLOCK_SHIFT) | sf))
+                if (bs, sname) == default:
+                    out.append((f"{name}/default", bf))
+                else:
+                    out.append((f"{name}/b{bs}/{sname}", bf | (code << _lib.OUT_BLOCK_SHIFT) | sf))
     return out
 
 

@@ -754,8 +754,8 @@ class _GPUPotBase:
         # The chunk layout and launch flags depend only on the call's shape, so they are
         # kept per shape on the object; the first chunk's copy-in is queued before the
         # tree's arguments at t are formed and the scratch they need is asked for (the
-        # host's remaining work before the first launch), so that copy overlaps it.  Each chunk then costs the
-        # host one C call and the first kernel follows its copy directly.
+        # host's remaining work before the first launch), so that copy overlaps it.  Each
+        # chunk then costs the host one C call and the first kernel follows its copy directly.
         prec = _PRECISIONS[self.precision or _default_precision]
         tuned = self.__dict__.get("_tuned") or {}
         key = (dev.index, mode, prec, n, chunk, self.binning, tuple(sorted(tuned.items())))
@@ -769,17 +769,19 @@ class _GPUPotBase:
             bounds = _chunk_bounds(n, chunk, wave)
             sizes = sorted({hi - lo for lo, hi in bounds})
             flags = {m: self._flags(mode, prec, m) for m in sizes}
+            # chunks in whole waves: one resident block per slot, so every thread of a launch
+            # takes the same number of passes (unless a tuned shape is set; a chunk of one
+            # wave takes one pass in any case)
+            grid1 = {}
             if wave and len(bounds) > 2 and all((hi - lo) % wave == 0 for lo, hi in bounds[:-1]):
-                # chunks in whole waves: one resident block per slot, so every thread of
-                # a launch takes the same number of passes (unless a tuned shape is set)
-                flags = {m: f if (f >> _lib.OUT_GRID_SHIFT) & 15 or (f >> _lib.OUT_PPT_SHIFT) & 15
-                         else f | (1 << _lib.OUT_GRID_SHIFT) for m, f in flags.items()}
+                grid1 = {m: 1 << _lib.OUT_GRID_SHIFT for m, f in flags.items() if m > wave
+                         and not ((f >> _lib.OUT_GRID_SHIFT) & 15 or (f >> _lib.OUT_PPT_SHIFT) & 15)}
             # the device buffers hold the largest chunk
-            plan = (bounds, max(sizes), flags)
+            plan = (bounds, max(sizes), flags, grid1)
             if len(plans) >= 64:
                 plans.clear()
             plans[key] = plan
-        bounds, chunk, flags = plan
+        bounds, chunk, flags, grid1 = plan
         ptr = lambda a: None if a is None else a.data_ptr()  # noqa: E731
         cur = torch.cuda.current_stream(dev)
         s_in, s_cmp, s_out = pipe["streams"]
@@ -793,6 +795,11 @@ class _GPUPotBase:
             ev_in[0].record(s_in)
         if cargs is None:
             cargs = self._c_args(t, dev)
+        kinds = {c.kind for c in cargs[0]}
+        if prec == _lib.PREC_MIXED or _lib.KIND_MULTIPOLE in kinds or _lib.KIND_CYLSPLINE not in kinds:
+            flags = {m: f | grid1.get(m, 0) for m, f in flags.items()}
+        # else the kernel for CylSplines, which takes one block per slot by itself and which a
+        # launch shape would rule out (1M points of a disk: 146 us, 284 with the shape)
         # the leaves at t decide which chunks sort
         nws = max(int(_lib.lib.agb_eval_scratch_bytes(*cargs, m, mode, prec, f))
                   for m, f in flags.items())
