@@ -280,6 +280,14 @@ def last_error() -> str:
     return lib.agb_last_error().decode()
 
 
+def raw_stream(dev) -> int:
+    """The cudaStream_t of the device's current torch stream (0.1 us where torch gives the number
+    itself, some 3 us through a Stream object)."""
+    import torch
+    get = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return get(dev.index) if get is not None else torch.cuda.current_stream(dev).cuda_stream
+
+
 def check(rc: int, what: str) -> None:
     if rc != AGB_OK:
         raise RuntimeError(f"{what} failed ({rc}): {last_error()}")

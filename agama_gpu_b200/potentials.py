@@ -461,7 +461,7 @@ class _GPUPotBase:
         if n == 0:
             return phi, grad, hess, rho
         ptr = lambda a: None if a is None else a.data_ptr()  # noqa: E731
-        stream = torch._C._cuda_getCurrentRawStream(dev.index)     # 0.1 us, a Stream object 2.2
+        stream = _lib.raw_stream(dev)
         flags = self._flags(mode, prec, n)
         ws, nws = self._workspace(cargs, n, dev, flags, mode, prec)
         rc = _lib.lib.agb_eval_ws(*cargs, arr.data_ptr(), n, mode, prec, ptr(phi), ptr(grad),
