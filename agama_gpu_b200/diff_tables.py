@@ -196,11 +196,12 @@ def multipole_consts_from_nodes(tables, phi: torch.Tensor, dphi_dr: torch.Tensor
     return torch.stack([q if torch.is_tensor(q) else zero + q for q in parts]).to(phi.device)
 
 
-def _power_slope(A: float, dA, lnr: float):
+def _power_slope(A, dA, lnr):
     """s = (A - W(A e^A)) / lnr of the builder's power-law fits with its derivatives."""
     from scipy.special import lambertw
-    ea = float(np.exp(A))
-    w = float(np.real(lambertw(A * ea, k=0 if A > -1.0 else -1)))
+    num = type(A)
+    ea = num(np.exp(A))
+    w = num(np.real(lambertw(A * ea, k=0 if A > -1.0 else -1)))
     ds = (1.0 - w / (A * ea * (1.0 + w)) * ea * (1.0 + A)) / lnr
     return (A - w) / lnr, [ds * q for q in dA]
 
@@ -208,14 +209,23 @@ def _power_slope(A: float, dA, lnr: float):
 def consts_and_jacobian(tables, p0: np.ndarray, d0: np.ndarray):
     """``multipole_consts_from_nodes`` in plain numbers, with its derivatives: (8,) values and
     (8, 6), the columns d/dPhi_00 at the nodes 0, 1, n-2, n-1 and d/d(dPhi_00/dr) at the nodes
-    0 and n-1, from the l=0 node values p0 and dPhi/dr d0 (nR,)."""
+    0 and n-1, from the l=0 node values p0 and dPhi/dr d0 (nR,).  Degenerate values divide by
+    zero as tensors do: to an infinity or NaN."""
+    try:
+        return _consts_and_jacobian(tables, p0, d0, float)       # 18 us less than as NumPy scalars
+    except ZeroDivisionError:
+        with np.errstate(all="ignore"):
+            return _consts_and_jacobian(tables, p0, d0, np.float64)
+
+
+def _consts_and_jacobian(tables, p0: np.ndarray, d0: np.ndarray, num):
     r = np.asarray(tables.r_grid, dtype=np.float64)
     v, J = np.zeros(8), np.zeros((8, 6))
     tiny = 100.0 * _EPS
     # inner fit: columns (P1, P2, d1) = (0, 1, 4)
-    P1, P2, d1, d2 = float(p0[0]), float(p0[1]), float(d0[0]), float(d0[1])
-    r1, r2 = float(r[0]), float(r[1])
-    lnr = float(np.log(r2 / r1))
+    P1, P2, d1, d2 = num(p0[0]), num(p0[1]), num(d0[0]), num(d0[1])
+    r1, r2 = num(r[0]), num(r[1])
+    lnr = num(np.log(r2 / r1))
     g1 = r1 * d1
     v[3], J[3, 0] = P1, 1.0
     A = np.inf
@@ -233,7 +243,7 @@ def consts_and_jacobian(tables, p0: np.ndarray, d0: np.ndarray):
             dU = [-U / s * q for q in ds]
             dU[2] += r1 / s
             dW = [(1.0 if i == 0 else 0.0) - q for i, q in enumerate(dU)]
-            pred_pow = U * s * float(np.exp(s * lnr)) / r2
+            pred_pow = U * s * num(np.exp(s * lnr)) / r2
         else:
             U, W, dU, dW = g1, P1, [0.0, 0.0, r1], [1.0, 0.0, 0.0]
             pred_pow = g1 / r2
@@ -252,11 +262,11 @@ def consts_and_jacobian(tables, p0: np.ndarray, d0: np.ndarray):
                 v[0] = inv
                 J[0, at] = [-inv * inv * q for q in dW]
     # outer fit in (eps, T, S): columns (P1, P2, d1) = (3, 2, 5)
-    P1, P2, d1 = float(p0[-1]), float(p0[-2]), float(d0[-1])
-    r1, r2 = float(r[-1]), float(r[-2])
-    lnr = float(np.log(r2 / r1))
+    P1, P2, d1 = num(p0[-1]), num(p0[-2]), num(d0[-1])
+    r1, r2 = num(r[-1]), num(r[-2])
+    lnr = num(np.log(r2 / r1))
     at = [3, 2, 5]
-    num1, num2, den1, den2 = r1 * d1, -P1, P1, P2 * float(np.exp(lnr))
+    num1, num2, den1, den2 = r1 * d1, -P1, P1, P2 * num(np.exp(lnr))
     roundoff = (abs(num1 - num2) < max(abs(num1), abs(num2)) * tiny or
                 abs(den1 - den2) < max(abs(den1), abs(den2)) * tiny)
     A = np.inf
@@ -270,7 +280,7 @@ def consts_and_jacobian(tables, p0: np.ndarray, d0: np.ndarray):
     if abs(A + 1.0) >= np.sqrt(_EPS):
         N, D = num1 - num2, den1 - den2
         s, ds = _power_slope(A, (lnr * (1.0 / D - N / (D * D)),
-                                 lnr * N * float(np.exp(lnr)) / (D * D), lnr * r1 / D), lnr)
+                                 lnr * N * num(np.exp(lnr)) / (D * D), lnr * r1 / D), lnr)
         s -= 1.0
     if not np.isfinite(s) or s >= 0.0:
         s, ds = -2.0, [0.0, 0.0, 0.0]
@@ -285,17 +295,61 @@ def consts_and_jacobian(tables, p0: np.ndarray, d0: np.ndarray):
     return v, J
 
 
+def _on_device(tables, dev: torch.device):
+    """The tables' grid and node values (r, phi, dphi) on the device.  Copying them waits for the
+    stream (a node fit of 200003 points takes 676 us with the copies in every pass, 403 without),
+    so the copies are kept beside host ones and made again when the values differ; each stream
+    has its own."""
+    from ._lib import raw_stream
+    now = [np.ascontiguousarray(a, dtype=np.float64)
+           for a in (tables.r_grid, tables.node_phi, tables.node_dphi_dr)]
+    held = tables.__dict__.setdefault("_on_device", {})
+    key = (dev.index, raw_stream(dev))
+    values = [(a.shape, a.tobytes()) for a in now]
+    had = held.get(key)
+    if had is not None and values == had[0]:
+        return had[1]
+    if len(held) >= 8:
+        held.clear()
+    copies = [torch.tensor(a, device=dev) for a in now]
+    held[key] = (values, copies)
+    return copies
+
+
+def _has_storage(*tensors) -> bool:
+    """Whether these are plain tensors in memory (not those of vmap, tracing and the like)."""
+    try:
+        return all(t.data_ptr() is not None for t in tensors)
+    except RuntimeError:
+        return False
+
+
+def _node_vjp_fits(tables, grad_poly: torch.Tensor, nodes, grad_const) -> bool:
+    """Whether the GPU kernel takes these: CUDA gradients, its number of nodes, and tensors of
+    exactly the shapes that it reads (what else there is, is left to torch)."""
+    from ._lib import NODE_VJP_MAX, MP_NCONST
+    if grad_poly.device.type != "cuda" or tables.resampled:
+        return False
+    if tables.node_phi is None or tables.node_dphi_dr is None:
+        return False
+    phi, dphi = (tables.node_phi, tables.node_dphi_dr) if nodes is None else nodes
+    n = int(np.asarray(tables.r_grid).size)
+    if not 2 <= n <= NODE_VJP_MAX or len(phi.shape) != 2 or phi.shape[0] != n or phi.shape[1] < 1:
+        return False
+    if tuple(dphi.shape) != tuple(phi.shape) or tuple(grad_poly.shape) != (phi.shape[1], n - 1, 6):
+        return False
+    if grad_const is not None and tuple(grad_const.shape) != (MP_NCONST,):
+        return False
+    given = [grad_poly] + ([] if nodes is None else list(nodes)) + ([] if grad_const is None else [grad_const])
+    return _has_storage(*given)
+
+
 def _node_vjp_cuda(tables, grad_poly: torch.Tensor, nodes, grad_const: Optional[torch.Tensor]):
     """(dL/dPhi, dL/d(dPhi/dr)) in the builder's order by the transposed builder on the GPU
-    (agb_multipole_node_vjp)."""
+    (agb_multipole_node_vjp); arguments as _node_vjp_fits has them."""
     from . import _lib
     dev = grad_poly.device
-    # the builder's own node tables, once per device
-    held = tables.__dict__.setdefault("_on_device", {})
-    if dev not in held:
-        held[dev] = [torch.tensor(np.ascontiguousarray(a), dtype=torch.float64, device=dev)
-                     for a in (tables.r_grid, tables.node_phi, tables.node_dphi_dr)]
-    r, phi, dphi = held[dev]
+    r, phi, dphi = _on_device(tables, dev)
     if nodes is not None:
         phi, dphi = (q.detach().to(dev, torch.float64).contiguous() for q in nodes)
     inv, jac, gc = float(tables.invPhi0), None, None
@@ -317,7 +371,7 @@ def _node_vjp_cuda(tables, grad_poly: torch.Tensor, nodes, grad_const: Optional[
             phi.shape[0], phi.shape[1], int(bool(tables.log_scaling)), float(tables.dlogr), inv,
             g.data_ptr(), r.data_ptr(), phi.data_ptr(), dphi.data_ptr(),
             None if gc is None else gc.data_ptr(), None if jac is None else jac.ctypes.data,
-            out[0].data_ptr(), out[1].data_ptr(), torch.cuda.current_stream(dev).cuda_stream)
+            out[0].data_ptr(), out[1].data_ptr(), _lib.raw_stream(dev))
     _lib.check(rc, "agb_multipole_node_vjp")
     return out[0], out[1]
 
@@ -394,8 +448,7 @@ def node_vjp(tables, grad_poly: torch.Tensor, n_file_cols: Optional[int],
     set_node_tables rebuilds them), without it they are held fixed.
     """
     dev = grad_poly.device
-    from ._lib import NODE_VJP_MAX
-    if dev.type == "cuda" and 2 <= tables.n_int + 1 <= NODE_VJP_MAX and not tables.resampled:
+    if _node_vjp_fits(tables, grad_poly, nodes, grad_const):
         gphi, gdphi = _node_vjp_cuda(tables, grad_poly, nodes, grad_const)
     else:
         gphi, gdphi = _node_vjp_torch(tables, grad_poly, nodes, grad_const)

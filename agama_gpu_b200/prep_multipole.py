@@ -58,6 +58,10 @@ class MultipoleTables:
     node_cols: np.ndarray = None     # (n_lm,) column of each harmonic in the coefficient file
     resampled: bool = False          # the input grid was not log-uniform and was resampled
 
+    def __getstate__(self):
+        """Copies and pickles carry the arrays, not what diff_tables keeps on the device."""
+        return {k: v for k, v in self.__dict__.items() if k != "_on_device"}
+
     @property
     def n_lm(self) -> int:
         return int(self.poly.shape[0])
