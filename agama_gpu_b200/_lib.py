@@ -10,6 +10,8 @@ import ctypes
 import struct
 from pathlib import Path
 
+import torch
+
 LIB_PATH = Path(__file__).resolve().parent / "libagb.so"
 
 AGB_OK = 0
@@ -283,7 +285,6 @@ def last_error() -> str:
 def raw_stream(dev) -> int:
     """The cudaStream_t of the device's current torch stream (0.1 us where torch gives the number
     itself, some 3 us through a Stream object)."""
-    import torch
     get = getattr(torch._C, "_cuda_getCurrentRawStream", None)
     return get(dev.index) if get is not None else torch.cuda.current_stream(dev).cuda_stream
 

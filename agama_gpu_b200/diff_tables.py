@@ -298,21 +298,20 @@ def _consts_and_jacobian(tables, p0: np.ndarray, d0: np.ndarray, num):
 def _on_device(tables, dev: torch.device):
     """The tables' grid and node values (r, phi, dphi) on the device.  Copying them waits for the
     stream (a node fit of 200003 points takes 676 us with the copies in every pass, 403 without),
-    so the copies are kept beside host ones and made again when the values differ; each stream
-    has its own."""
+    so the copies are kept beside host ones and made again when the values differ (a comparison
+    of 10 us at lmax 12, 40 at lmax 32); each stream has its own."""
     from ._lib import raw_stream
     now = [np.ascontiguousarray(a, dtype=np.float64)
            for a in (tables.r_grid, tables.node_phi, tables.node_dphi_dr)]
     held = tables.__dict__.setdefault("_on_device", {})
     key = (dev.index, raw_stream(dev))
-    values = [(a.shape, a.tobytes()) for a in now]
     had = held.get(key)
-    if had is not None and values == had[0]:
+    if had is not None and all(a.shape == b.shape and (a == b).all() for a, b in zip(now, had[0])):
         return had[1]
     if len(held) >= 8:
         held.clear()
     copies = [torch.tensor(a, device=dev) for a in now]
-    held[key] = (values, copies)
+    held[key] = ([a.copy() for a in now], copies)
     return copies
 
 
