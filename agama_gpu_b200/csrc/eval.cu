@@ -526,7 +526,8 @@ static size_t ws_bound(const agb_component* comps, int n_comps, int64_t n, int o
 }
 
 // Calls below AGB_BIN_MIN_POINTS need no scratch: given less than the sort takes, they are
-// evaluated in input order (each point's result is the same).
+// evaluated in input order (each point's result is the same).  agb_eval_static's shared array
+// is not used for them either, so that small calls may overlap on the GPU.
 static bool sort_optional(int64_t n, int out_flags)
 {
     return n < AGB_BIN_MIN_POINTS && !(out_flags & AGB_OUT_BIN_ALWAYS);
@@ -683,7 +684,7 @@ static int eval_impl(const agb_component* comps, int n_comps, const agb_leaf* le
 
     BinPlan b = plan_binning(comps, leaves, n_leaves, n, out_flags, 1, mode, precision);
     if (sort_optional(n, out_flags) &&
-        (own_ws || !workspace || ((uintptr_t)workspace & 255u) || workspace_bytes < ws_bytes(b, n)))
+        (own_ws || fixed_ws || !workspace || ((uintptr_t)workspace & 255u) || workspace_bytes < ws_bytes(b, n)))
         b.on = false;
     // sorted-order output staging when the workspace has room for it (always for
     // agb_eval's own allocation and for workspaces sized by agb_eval_workspace_bytes)

@@ -33,6 +33,10 @@ def _tree(name):
         return _halo(12) + agb.CylSplinePotentialGPU(bar_cylspline())
     if name == "disk":
         return agb.CylSplinePotentialGPU(bar_cylspline()) + mn
+    if name == "moving_disk":
+        t = np.arange(5.0)
+        return mn + agb.ShiftedPotentialGPU(agb.CylSplinePotentialGPU(bar_cylspline()),
+                                            np.column_stack([0.7 * t, np.sin(t), 0.1 * t * t, t]))
     # snapshots of unequal orders: the components in use change with time
     return mn + agb.EvolvingPotentialGPU([_halo(4, seed=1), _halo(12, seed=2), _halo(32, seed=3)],
                                          [0.0, 1.0, 2.0])
@@ -78,9 +82,10 @@ def test_every_kernel_gives_the_same_bits(name, prec):
 
 
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
-def test_leaves_from_the_device_give_the_same_bits(prec):
+@pytest.mark.parametrize("name", ["snapshots", "moving_disk"])
+def test_leaves_from_the_device_give_the_same_bits(name, prec):
     from agama_gpu_b200 import _lib
-    pot = _tree("snapshots")
+    pot = _tree(name)
     for n in (100, 3001, 20011):
         x = _points(n)
         for t in (0.0, 0.3, 1.0, 1.9, 2.5):

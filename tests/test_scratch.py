@@ -147,3 +147,27 @@ def test_default_call_is_no_slower_than_one_thread_per_point(tree, n, prec):
         return best
     time(0)
     assert time(0) < 1.25 * time(_lib.OUT_BIN_ALWAYS | 2 << _lib.OUT_GRID_SHIFT)
+
+
+@pytest.mark.gpu
+def test_small_static_calls_may_overlap():
+    """agb_eval_static's shared array is not used below the documented size: small calls on two
+    streams at the same time give their own results."""
+    import torch
+    from agama_gpu_b200 import _lib
+    from agama_gpu_b200.synthetic import hernquist_points
+    pots = [_multipole(32, nodes=100), _multipole(24, 4, 60)]
+    xs = [torch.from_numpy(hernquist_points(n, 10.0, n)).cuda() for n in (16383, 9001)]
+    cargs = [p._c_args(0.0, x.device) for p, x in zip(pots, xs)]
+    out = [[torch.empty_like(x) for _ in range(10)] for x in xs]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for k in range(10):
+        for i in (0, 1):
+            assert _lib.lib.agb_eval_static(*cargs[i], xs[i].data_ptr(), xs[i].shape[0], _lib.MODE_GRAD,
+                                            0, None, out[i][k].data_ptr(), None, None, _lib.OUT_NEGATE,
+                                            streams[i].cuda_stream) == 0
+    torch.cuda.synchronize()
+    for p, x, fs in zip(pots, xs, out):
+        ref = p.force(x)
+        assert all(torch.equal(f, ref) for f in fs)
