@@ -85,7 +85,7 @@ __device__ __forceinline__ void mp_group(const R* rec, int m, int lmax, R s, dou
     const int ts = m * AGB_SKIP_N;
     auto skip2 = [&](int L) {
         const auto ab = MPConst<R>::skip(ts + (L >> 1));
-        const R t = c2 + (R)ab.x;
+        const R t = mp_cos2_add<MODE, R>(cth, c2, (R)ab.x);
         const R Pn = fma(t, Pc, (R)ab.y * Pp);
         if (NEED_ANG) {
             const R dPn = fma(w2, Pc, fma(t, dPc, (R)ab.y * dPp));

@@ -402,6 +402,17 @@ __device__ __forceinline__ void mp_col_finish(MPCol<R>& g, R inv_sth, R q1, R np
         g.VRR *= R(2);                                          // the joint pass sums C''/2
 }
 
+// cos^2(theta) + A_l of the two-step walk, c2 the rounded square.  FP64 forces and densities
+// round once, and the square needs no register of its own (4M-point composite, forces 6.65 ->
+// 6.57 ms); potentials, with registers to spare, are slower so (5.23 -> 5.27), Hessians equal.
+template <int MODE, typename R>
+__device__ __forceinline__ R mp_cos2_add(R cth, R c2, R a)
+{
+    if (std::is_same<R, double>::value && (MODE == AGB_MODE_GRAD || MODE == AGB_MODE_DENS))
+        return fma(cth, cth, a);
+    return std::is_same<R, double>::value ? (R)__dadd_rn((double)c2, (double)a) : c2 + a;
+}
+
 // One |m| group's sums combined with cos/sin(m phi), and the rotation to the next m, with
 // their roundings spelled out (as in mp_hess_end below), so that the kernels that add the
 // groups (one thread per point, batches, a block per tile) round alike: a point's result does
@@ -442,7 +453,7 @@ __device__ __forceinline__ void mp_combine(MPSums& t, const MPCol<R>& gc, const 
                                            int m, double cm, double sm)
 {
     auto add = [](double& s, R c, R v, double tc, double ts) {
-        s = __dadd_rn(s, fma((double)v, ts, __dmul_rn((double)c, tc)));
+        s = __dadd_rn(s, fma((double)c, tc, __dmul_rn((double)v, ts)));
     };
     add(t.A, gc.V, gs.V, cm, sm);
     if (MODE != AGB_MODE_POT) add(t.B, gc.VR, gs.VR, cm, sm);
@@ -527,7 +538,7 @@ __device__ __forceinline__ void mp_harmonics_reg(const DevComp& c, int k, double
         const int ts = m * AGB_SKIP_N;
         auto skip2 = [&](int L) {
             const auto ab = MPConst<R>::skip(ts + (L >> 1));
-            const R t = c2 + (R)ab.x;
+            const R t = mp_cos2_add<MODE, R>(cth, c2, (R)ab.x);
             const R Pn = fma(t, Pc, (R)ab.y * Pp);
             if (NEED_ANG) {
                 const R dPn = fma(w2, Pc, fma(t, dPc, (R)ab.y * dPp));
@@ -648,7 +659,7 @@ __device__ __forceinline__ void mp_harmonics_reg2(const DevComp& c1, const DevCo
         const int ts = m * AGB_SKIP_N;
         auto skip2 = [&](int L) {
             const auto ab = MPConst<R>::skip(ts + (L >> 1));
-            const R t = cc2 + (R)ab.x;
+            const R t = mp_cos2_add<MODE, R>(cth, cc2, (R)ab.x);
             const R Pn = fma(t, Pc, (R)ab.y * Pp);
             if (NEED_ANG) {
                 const R dPn = fma(w2, Pc, fma(t, dPc, (R)ab.y * dPp));

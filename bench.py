@@ -57,9 +57,10 @@ def step_times(k_total: int):
 
 
 def flops_per_step(pot, xyz: np.ndarray, t: float) -> tuple:
-    """Algorithmic FLOPs of one Phi+F evaluation (the roofline's fixed convention):
-    Multipole 48*n_harm + 64 per point inside its grid (64 outside), analytic 30
-    per component.  Returns (fp32-eligible harmonic flops, fp64 flops)."""
+    """FLOPs of one Phi+F evaluation as the kernels execute them (a multiply-add is two):
+    Multipole 30*n_harm + 64 per point inside its grid (64 outside; per (l, |m|) pair 6
+    instructions of the recurrence, and per column 9 of the joint Horner pass and 3 of the
+    sums), analytic 30 per component.  Returns (fp32-eligible harmonic flops, fp64 flops)."""
     from agama_gpu_b200 import _lib as L
     f_harm = 0.0
     f_point = 0.0
@@ -69,7 +70,7 @@ def flops_per_step(pot, xyz: np.ndarray, t: float) -> tuple:
             x = sigma * xyz - np.asarray(gamma)[None, :]
             lr = np.log(np.maximum(np.linalg.norm(x, axis=1), 1e-300))
             inside = np.count_nonzero((lr >= tb.logr_min) & (lr < tb.logr_min + tb.n_int * tb.dlogr))
-            f_harm += 48.0 * tb.n_lm * inside
+            f_harm += 30.0 * tb.n_lm * inside
             f_point += 64.0 * len(xyz)
         elif comp.kind == L.KIND_CYLSPLINE:
             f_harm += 110.0 * comp.tables.n_harm * len(xyz)
@@ -278,7 +279,7 @@ def batched_units(dev, n_units: int, steps: int, warmup: int, lf_steps: int, pre
         units.append(mp)
         counts.append(n)
         xs.append(hernquist_points(n, spec["a"], 1000 + spec["index"]))
-        flops += n * (48.0 * mp.tables.n_lm + 64.0)
+        flops += n * (30.0 * mp.tables.n_lm + 64.0)
     batch = agb.BatchedPotentialGPU(units, counts, precision=precision)
     x = torch.from_numpy(np.concatenate(xs)).to(dev)
     del xs
@@ -702,7 +703,7 @@ def main():
             "bound": "fp32+fp64 pipes (mixed); fp64 pipe (plain)", "unit": "TFLOP/s",
             "note": "FP32/FP64 ALU-bound: the peaks are measured live (FMA chains) because the "
                     "pool's measured peaks cover only HBM copy and bf16 GEMM; flops count "
-                    "48 per harmonic per Multipole, the two Evolving snapshots each as if "
+                    "30 per harmonic per Multipole, the two Evolving snapshots each as if "
                     "walked alone (the mixed kernel shares their recurrences, ~2 % fewer "
                     "flops executed)",
             "achieved": achieved32, "peak": eff_peak32, "frac": achieved32 / eff_peak32,
