@@ -282,11 +282,15 @@ def last_error() -> str:
     return lib.agb_last_error().decode()
 
 
+_current_raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def raw_stream(dev) -> int:
     """The cudaStream_t of the device's current torch stream (0.1 us where torch gives the number
     itself, some 3 us through a Stream object)."""
-    get = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    return get(dev.index) if get is not None else torch.cuda.current_stream(dev).cuda_stream
+    if _current_raw is not None:
+        return _current_raw(dev.index)
+    return torch.cuda.current_stream(dev).cuda_stream
 
 
 def check(rc: int, what: str) -> None:

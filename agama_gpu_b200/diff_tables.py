@@ -339,12 +339,12 @@ def _node_vjp_fits(tables, grad_poly: torch.Tensor, nodes, grad_const) -> bool:
     if tables.node_phi is None or tables.node_dphi_dr is None:
         return False
     phi, dphi = (tables.node_phi, tables.node_dphi_dr) if nodes is None else nodes
-    n = int(np.asarray(tables.r_grid).size)
+    n = len(tables.r_grid)
     if not 2 <= n <= NODE_VJP_MAX or len(phi.shape) != 2 or phi.shape[0] != n or phi.shape[1] < 1:
         return False
-    if tuple(dphi.shape) != tuple(phi.shape) or tuple(grad_poly.shape) != (phi.shape[1], n - 1, 6):
+    if dphi.shape != phi.shape or grad_poly.shape != (phi.shape[1], n - 1, 6):
         return False
-    if grad_const is not None and tuple(grad_const.shape) != (MP_NCONST,):
+    if grad_const is not None and grad_const.shape != (MP_NCONST,):
         return False
     given = [grad_poly] + ([] if nodes is None else list(nodes)) + ([] if grad_const is None else [grad_const])
     return _has_storage(*given)
@@ -372,12 +372,15 @@ def _node_vjp_cuda(tables, grad_poly: torch.Tensor, nodes, grad_const: Optional[
         gc = grad_const.to(device=dev, dtype=torch.float64).contiguous()
     g = grad_poly.to(torch.float64).contiguous()
     out = torch.zeros((2,) + tuple(phi.shape), dtype=torch.float64, device=dev)
-    with torch.cuda.device(dev):
-        rc = _lib.lib.agb_multipole_node_vjp(
-            phi.shape[0], phi.shape[1], int(bool(tables.log_scaling)), float(tables.dlogr), inv,
+    args = (phi.shape[0], phi.shape[1], int(bool(tables.log_scaling)), float(tables.dlogr), inv,
             g.data_ptr(), r.data_ptr(), phi.data_ptr(), dphi.data_ptr(),
             None if gc is None else gc.data_ptr(), None if jac is None else jac.ctypes.data,
             out[0].data_ptr(), out[1].data_ptr(), _lib.raw_stream(dev))
+    if torch.cuda.current_device() == dev.index:
+        rc = _lib.lib.agb_multipole_node_vjp(*args)
+    else:
+        with torch.cuda.device(dev):
+            rc = _lib.lib.agb_multipole_node_vjp(*args)
     _lib.check(rc, "agb_multipole_node_vjp")
     return out[0], out[1]
 

@@ -540,7 +540,7 @@ class _GPUPotBase:
         gp = None if g_phi is None else g_phi.to(device=dev, dtype=torch.float64).contiguous()
         gf = None if g_force is None else g_force.to(device=dev, dtype=torch.float64).contiguous()
         ptr = lambda a: None if a is None else a.data_ptr()  # noqa: E731
-        stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+        stream = _lib.raw_stream(dev)
         for comp, sigma, gamma, ampl in fused:
             c = comp._device_component(dev)
             lf = _lib.AgbLeaf()

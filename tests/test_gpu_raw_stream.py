@@ -3,6 +3,7 @@ import pytest
 
 from agama_gpu_b200 import _lib
 
+
 @pytest.mark.gpu
 def test_stream_without_the_raw_number(monkeypatch):
     """A torch that does not give the stream's number itself: the same stream."""
@@ -19,6 +20,6 @@ def test_stream_without_the_raw_number(monkeypatch):
             want = _lib.raw_stream(dev)
             assert want == s.cuda_stream
             with monkeypatch.context() as m:
-                m.delattr(torch._C, "_cuda_getCurrentRawStream")
+                m.setattr(_lib, "_current_raw", None)
                 assert _lib.raw_stream(dev) == want
                 assert torch.equal(pot.force(x), ref)
