@@ -250,8 +250,8 @@ int agb_eval_ws(const agb_component* comps, int n_comps,
 
 /*
  * Points that one wave of the evaluator's resident threads holds on the current
- * device (SMs x resident blocks x 256) for the kernel this tree, mode and
- * precision select; 0 for bad arguments.  A call of n points with
+ * device (SMs x resident blocks x 256) for the one-thread-per-point kernel of this
+ * tree, mode and precision; 0 for bad arguments.  A call of n points with
  * AGB_OUT_GRID(1) takes ceil(n / wave) passes of its threads over the points, so
  * callers that split work into several calls (the pipelined host path) size the
  * calls in multiples of it.  No reference counterpart: the reference evaluates
