@@ -44,7 +44,7 @@ struct EvalArgs {
     int n_leaves;
     int out_flags;
     int soa;                 // 1: x, y, z separate arrays (kernel-signature entries)
-    int split_buf;           // agb_split_kernel: bytes of each of its two buffers of sums
+    int split_buf;           // agb_split_kernel: bytes of a buffer of the groups' shares
     long long chunk;         // points per block: block b evaluates [b*chunk, (b+1)*chunk)
     const double* xyz;       // AoS N x 3 when !soa (sorted copy when perm != null)
     const int* perm;         // binned order: point pos is input point perm[pos]

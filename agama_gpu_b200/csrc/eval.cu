@@ -423,19 +423,28 @@ struct BinPlan {
 // 1.06 (144, 1); with tables larger than the L1s 0.27 (153, 8), 1.2 (561, 8).  The potential
 // alone gains nearly twice as much, mixed precision a little less.  Multipoles in other frames
 // gain too, since the points of one interval lie together there as well (eight of lmax 8, each
-// in its own frame, 400003 points: 691 -> 513 us), and so do CylSplines, whose cells a warp's
-// points then share more often (13 harmonics beside a lmax-8 Multipole, 400003 points: forces
-// 341 -> 272 us, mixed 294 -> 251).
-static double sort_gain(const agb_component& c, int mode, int precision)
+// in its own frame, 400003 points: 691 -> 513 us), and in large calls so do CylSplines, whose
+// cells a warp's points then share more often: 300007 points, lmax 8 and 7 harmonics, FP64 forces
+// 195 -> 157 us of a sphere's points, 141 -> 125 of a disk's.  In mixed precision a disk's points
+// lose what a sphere's gain (7 harmonics 118 -> 129 and 164 -> 145); with the larger tables of
+// 13 harmonics little is lost and as much gained (157 -> 160 and 203 -> 182): the line lies
+// between, and for Hessians (7 harmonics FP64 196 -> 193 and 290 -> 232; mixed 205 -> 225 and 309
+// -> 264) as well.
+static double sort_gain(const agb_component& c, int64_t n, int mode, int precision)
 {
-    const bool hess = mode == AGB_MODE_HESS || mode == AGB_MODE_VJP || mode == AGB_MODE_VJPF;
-    if (c.kind == AGB_KIND_CYLSPLINE) return c.n_lm * (hess ? 0.027 : 0.008);
+    const bool mixed = precision == AGB_PREC_MIXED;
+    if (c.kind == AGB_KIND_CYLSPLINE) {
+        if (n <= AGB_BIN_SMALL) return 0.0;          // bound by latency: 50 -> 56 us sorted
+        if (mode == AGB_MODE_HESS || mode == AGB_MODE_VJP || mode == AGB_MODE_VJPF)
+            return 0.04 * std::max(0, c.n_lm - 4);
+        return mixed ? 0.0125 * std::max(0, c.n_lm - 5) : 0.008 * c.n_lm;
+    }
     if (c.kind != AGB_KIND_MULTIPOLE) return 0.0;
     int offsets = 8;
     for (int q = 8; q > 1 && (c.n_lm * 48 / 16) % (16 / q) == 0; q >>= 1) offsets = q / 2;
     const double l2 = 48.0 * c.n_lm * c.n_int > 400e3 ? 0.8e-3 : 0.0;
     return c.n_lm * (6.5e-3 / offsets + 0.5e-3 + l2) * (mode == AGB_MODE_POT ? 1.7 : 1.0) *
-           (precision == AGB_PREC_MIXED ? 0.8 : 1.0);
+           (mixed ? 0.8 : 1.0);
 }
 
 // Whether sorting n points pays: the sort and the gather of the outputs cost 13 us, or 5 us
@@ -478,7 +487,7 @@ static BinPlan plan_binning(const agb_component* comps, const agb_leaf* leaves, 
     b.one = n <= (eval ? AGB_BIN_SLICED : AGB_BIN_SMALL) && c.n_int + 2 <= AGB_BIN_SMALL_BINS;
     if (eval && !(out_flags & AGB_OUT_BIN_ALWAYS)) {
         double gain = 0.0;
-        for (int L = 0; L < n_leaves; ++L) gain += sort_gain(comps[leaves[L].comp], mode, precision);
+        for (int L = 0; L < n_leaves; ++L) gain += sort_gain(comps[leaves[L].comp], n, mode, precision);
         if (!sort_pays(gain, n, b.one && n <= AGB_BIN_SMALL, mode)) return b;
     }
     b.on = true;

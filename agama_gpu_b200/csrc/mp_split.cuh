@@ -22,6 +22,12 @@ __host__ __device__ constexpr int split_out(int mode)
     return mode == AGB_MODE_HESS ? 10 : mode == AGB_MODE_GRAD ? 4 : 1;
 }
 
+// bytes of a tile's results, 16-byte aligned
+__host__ __device__ constexpr int split_results(int mode, int T, int n_leaves)
+{
+    return (n_leaves * split_out(mode) * T * (int)sizeof(double) + 15) & ~15;
+}
+
 // most threads of a block: 128 registers a thread, 255 with Hessians
 __host__ __device__ constexpr int split_threads(int mode)
 {

@@ -6,9 +6,9 @@
 
 // A few points per block, the harmonics split over its warps (mp_split.cuh): calls too small
 // to fill the GPU with one thread per point.  Block b evaluates the tile of a.chunk <= 32
-// points from b * a.chunk on.  Dynamic shared memory: two buffers of a.split_buf bytes with the
-// |m| groups' shares of the sums [m][sum][point] (Hessians: their columns), then every leaf's
-// results [leaf][value][point].
+// points from b * a.chunk on.  Dynamic shared memory: every leaf's results [leaf][value][point],
+// then a buffer of a.split_buf bytes with the |m| groups' shares of the sums [m][sum][point]
+// (Hessians: their columns), and another one where several leaves are walked.
 template <int MODE, typename R, bool DYN>
 __global__ void __launch_bounds__(split_threads(MODE), 1)
 agb_split_kernel(const __grid_constant__ EvalArgs a)
@@ -27,7 +27,8 @@ agb_split_kernel(const __grid_constant__ EvalArgs a)
     const int T = (int)a.chunk;
     const long long pos = (long long)blockIdx.x * T + lane;
     const bool live = lane < T && pos < a.n;
-    double* res = reinterpret_cast<double*>(split_smem + 2 * a.split_buf);
+    double* res = reinterpret_cast<double*>(split_smem);
+    char* bufs = split_smem + split_results(CM, T, a.n_leaves);
     double x = 0.0, y = 0.0, z = 0.0;
     if (live) {
         if (a.soa) {
@@ -48,7 +49,7 @@ agb_split_kernel(const __grid_constant__ EvalArgs a)
         bool mine, grid = false;
         int k = 0;
         double s = 0.0, inv_r = 0.0, Rc = 0.0, cth = 1.0, sth = 0.0, cph = 1.0, sph = 0.0;
-        char* buf = split_smem + (turn & 1) * a.split_buf;
+        char* buf = bufs + (turn & 1) * a.split_buf;
         double* sums = reinterpret_cast<double*>(buf) + lane;
         R* cols = reinterpret_cast<R*>(buf) + lane;
         if (walked) {
@@ -136,8 +137,8 @@ agb_split_kernel(const __grid_constant__ EvalArgs a)
     eval_write<MODE>(a, pos, a.perm ? (long long)a.perm[pos] : pos, phi, g0, g1, g2, h, rho);
 }
 
-// dynamic shared memory of a block: lmax 32 with Hessians in FP64 needs 203 KB of columns, and
-// 2.5 KB per leaf of results (larger trees take one thread per point there)
+// dynamic shared memory of a block: two leaves of lmax 32 with Hessians in FP64 need 203 KB of
+// columns, and 2.5 KB per leaf of results (larger trees take one thread per point there)
 #define AGB_SPLIT_SMEM (220 * 1024)
 
 // What a call's leaves cost a warp, in units of the latency of one (l, |m|) step.
@@ -244,7 +245,9 @@ static bool split_shape(EvalArgs& a, int& S, int& T, size_t& smem)
     a.split_buf = T * (work.lmax + 1) * (HESS ? AGB_SPLIT_HESS_COLS * (int)sizeof(R)
                                               : split_sums(CM) * (int)sizeof(double));
     a.split_buf = (a.split_buf + 15) & ~15;
-    smem = 2 * (size_t)a.split_buf + sizeof(double) * T * (size_t)a.n_leaves * split_out(CM);
+    // leaves from the device may be walked or not, as their component at that time is
+    const int buffers = work.walked > 1 || a.dleaves ? 2 : 1;
+    smem = buffers * (size_t)a.split_buf + split_results(CM, T, a.n_leaves);
     if (smem > AGB_SPLIT_SMEM) return false;
     const int fit = std::max(1, 228 * 1024 / ((int)smem + 1024));
     auto per_sm = [&](long long tile) { return ((a.n + tile - 1) / tile + sms - 1) / sms; };
