@@ -27,6 +27,7 @@ OUT_BLOCK_SHIFT = 12
 OUT_PPT_SHIFT = 16
 MP_NCONST = 8                # agb_component.p[3..9] + pad: invPhi0, inner s U W, outer s U W
 BIN_MIN_POINTS = 16384
+SORT_NEVER = 346         # points x leaves up to which no evaluation sorts by itself (sort_pays)
 NODE_VJP_MAX = 256
 
 KIND_MULTIPOLE = 1

@@ -434,6 +434,8 @@ class _GPUPotBase:
         return f
 
     def _workspace(self, cargs, n: int, dev: torch.device, flags: int, mode: int, prec: int):
+        if n * cargs[3] <= _lib.SORT_NEVER and not flags & _lib.OUT_BIN_ALWAYS:
+            return None, 0              # what the library would answer (a call of one point 17.3 -> 15.7 us)
         nws = int(_lib.lib.agb_eval_scratch_bytes(*cargs, n, mode, prec, flags))
         return (torch.empty(nws, dtype=torch.uint8, device=dev) if nws else None), nws
 

@@ -39,6 +39,19 @@ def test_workspace_of_the_largest_call_serves_smaller_ones(lmax):
     assert _lib.lib.agb_eval_scratch_bytes(*two, 10**6, _lib.MODE_POT, 0, _lib.OUT_NO_BINNING) == 0
 
 
+def test_fewest_points_never_sort():
+    """The calls for which no scratch is asked (SORT_NEVER) are calls that need none."""
+    from agama_gpu_b200 import _lib
+    from itertools import product
+    for columns, leaves in product((45, 64, 144, 560, 561, 1024, 1088, 1089), (1, 2, 7, _lib.MAX_LEAVES)):
+        args = _descriptors(columns, nodes=200, n_leaves=leaves)
+        for mode, prec in product(range(5), (_lib.PREC_FP64, _lib.PREC_MIXED)):
+            for n in {1, _lib.SORT_NEVER // leaves}:
+                assert _lib.lib.agb_eval_scratch_bytes(*args, n, mode, prec, 0) == 0
+                # by flag they do
+                assert _lib.lib.agb_eval_scratch_bytes(*args, n, mode, prec, _lib.OUT_BIN_ALWAYS) > 0
+
+
 def _multipole(lmax, seed=3, nodes=50):
     import agama_gpu_b200 as agb
     from agama_gpu_b200.synthetic import nfw_multipole
